@@ -4,7 +4,6 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <vector>
 
 #include "common.cuh"
 #include "context.cuh"
@@ -62,24 +61,6 @@ static void toric_matrix(uint8_t out[kN * kN]) {
   for (int i = 0; i < kN; ++i)
     for (int j = 0; j < kN; ++j)
       out[i * kN + j] = gf8_mul_c(pw(uint8_t(1 + j / 7), i / 7), pw(uint8_t(1 + j % 7), i % 7));
-}
-
-// GL2(F7) as permutations of the 49 points, matrices (a b; c d) in the
-// lexicographic order of (a, b, c, d) with nonzero determinant; point (x, y)
-// maps to (a x + b y, c x + d y) (champion_search_canonical.py:61-74).
-static void gl2_table(uint8_t out[kGl2Order * kN]) {
-  int m = 0;
-  for (int a = 0; a < 7; ++a)
-    for (int b = 0; b < 7; ++b)
-      for (int c = 0; c < 7; ++c)
-        for (int d = 0; d < 7; ++d) {
-          if (((a * d - b * c) % 7 + 7) % 7 == 0) continue;
-          for (int p = 0; p < kN; ++p) {
-            const int x = p / 7, y = p % 7;
-            out[m * kN + p] = uint8_t(((a * x + b * y) % 7) * 7 + (c * x + d * y) % 7);
-          }
-          ++m;
-        }
 }
 
 }  // namespace tg
@@ -167,8 +148,6 @@ int tg_context_create(int device, const int32_t* h_M, tg_context** out_ctx) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetDeviceProperties");
   uint8_t T[kN * kN];
   toric_matrix(T);
-  std::vector<uint8_t> gl2(size_t(kGl2Order) * kN);
-  gl2_table(gl2.data());
   tg_context* ctx = new tg_context();
   ctx->device = device;
   ctx->sm_count = prop.multiProcessorCount;
@@ -182,14 +161,11 @@ int tg_context_create(int device, const int32_t* h_M, tg_context** out_ctx) {
         planes[r * 3 + b] |= uint64_t((M[r * kN + j] >> b) & 1u) << j;
   e = cudaMalloc(&ctx->d_M, sizeof(M));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_Mp, sizeof(planes));
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_gl2, gl2.size());
   if (e == cudaSuccess) e = cudaMemcpy(ctx->d_M, M, sizeof(M), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(ctx->d_Mp, planes, sizeof(planes), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(ctx->d_gl2, gl2.data(), gl2.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     if (ctx->d_M) cudaFree(ctx->d_M);
     if (ctx->d_Mp) cudaFree(ctx->d_Mp);
-    if (ctx->d_gl2) cudaFree(ctx->d_gl2);
     delete ctx;
     return cuda_fail(e, "context tables");
   }
@@ -202,7 +178,6 @@ int tg_context_destroy(tg_context* ctx) {
   DeviceGuard g(ctx->device);
   if (ctx->d_M) cudaFree(ctx->d_M);
   if (ctx->d_Mp) cudaFree(ctx->d_Mp);
-  if (ctx->d_gl2) cudaFree(ctx->d_gl2);
   delete ctx;
   return TG_OK;
 }
@@ -317,7 +292,6 @@ static int bind_distance(tg_context* ctx, const tg_distance_params* p, const int
   a.seed = p->sample_seed;
   a.tab.M = ctx->d_M;
   a.tab.Mp = ctx->d_Mp;
-  a.tab.gl2 = ctx->d_gl2;
   a.is_toric = ctx->is_toric;
   a.is_blocks_per_sm = p->is_blocks_per_sm > 0 ? p->is_blocks_per_sm : 5;
   // defaults: the shape the tuner picks for k = 14, the largest codes of a
@@ -590,7 +564,7 @@ int tg_canonical_sets(tg_context* ctx, const int32_t* d_sets, int32_t n, int32_t
   DeviceGuard g(ctx->device);
   if (g.error() != cudaSuccess) return cuda_fail(g.error(), "cudaSetDevice");
   static const int32_t kDummy = 0;
-  return run_canonical(ctx->device, ctx->sm_count, ctx->d_gl2, k > 0 ? d_sets : &kDummy, nullptr,
+  return run_canonical(ctx->sm_count, k > 0 ? d_sets : &kDummy, nullptr,
                        n, k, d_out_mask, d_out_key_lo, d_out_key_hi, d_status,
                        static_cast<cudaStream_t>(stream));
 }
@@ -603,7 +577,7 @@ int tg_canonical_masks(tg_context* ctx, const uint64_t* d_masks, int32_t n, uint
   if (!d_masks || !d_out_mask) return invalid("tg_canonical_masks: NULL device pointer");
   DeviceGuard g(ctx->device);
   if (g.error() != cudaSuccess) return cuda_fail(g.error(), "cudaSetDevice");
-  return run_canonical(ctx->device, ctx->sm_count, ctx->d_gl2, nullptr, d_masks, n, 0, d_out_mask,
+  return run_canonical(ctx->sm_count, nullptr, d_masks, n, 0, d_out_mask,
                        d_out_key_lo, d_out_key_hi, nullptr, static_cast<cudaStream_t>(stream));
 }
 
@@ -616,7 +590,7 @@ int tg_expand_canonical(tg_context* ctx, const uint64_t* d_parents, int32_t n, u
   if (!d_parents || !d_out) return invalid("tg_expand_canonical: NULL device pointer");
   DeviceGuard g(ctx->device);
   if (g.error() != cudaSuccess) return cuda_fail(g.error(), "cudaSetDevice");
-  return run_canonical(ctx->device, ctx->sm_count, ctx->d_gl2, nullptr, d_parents, n * kN, 0,
+  return run_canonical(ctx->sm_count, nullptr, d_parents, n * kN, 0,
                        d_out, nullptr, nullptr, nullptr, static_cast<cudaStream_t>(stream), 1);
 }
 

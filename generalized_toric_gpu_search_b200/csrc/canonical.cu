@@ -7,25 +7,19 @@
 // per index with the largest index most significant.  For sets of equal size
 // that order is the order of 49-bit masks (bit i = exponent index i), so the
 // key is the smallest mask among the AGL2 images of S that contain the origin.
-// This file computes that mask for any popcount 1..49 and derives the
-// reference's packed 128-bit key from it for k <= 16.
-//
-// Kernel: one warp per set, persistent CTAs; the 2016 x 49 point permutation
-// table of GL2(F7) (98,784 bytes) sits in shared memory.  Lane l handles the
-// matrices l, l + 32, ...: it maps the mask point by point, then for every
-// point q of the image translates the image by -q on the torus Z_7^2
-// (a per-row 7-bit rotation followed by a 49-bit rotation by 7 rows) and keeps
-// the smallest mask, skipping the translations whose top row already exceeds
-// the best (canon_mask_warp_min in common.cuh).  A 64-bit warp min-reduction
-// finishes the set.
+// This file computes that mask for any popcount 1..49 (canon_form.cuh) and
+// derives the reference's packed 128-bit key from it for k <= 16.
 #include "common.cuh"
+#include "canon_form.cuh"
 #include "canonical.cuh"
 
 namespace tg {
 
-constexpr int kCanonTPB = 512;                     // 2 CTAs per SM: 32 warps
-constexpr int kGl2Row = 52;                        // padded row in shared memory
-constexpr int kGl2SharedBytes = kGl2Order * kGl2Row;  // 104,832
+// 16 sets per CTA (8 lanes each): 64 sets already spread over 4 SMs, and the
+// tables and lists take 8 KB of shared memory, so registers bound the
+// occupancy.
+constexpr int kCanonTPB = 128;
+constexpr int kCanonSets = kCanonTPB / 8;
 
 struct CanonArgs {
   const int32_t* sets;    // (n, k) rows, or NULL
@@ -37,83 +31,78 @@ struct CanonArgs {
   uint64_t* out_lo;
   uint64_t* out_hi;
   int32_t* status;
-  const uint8_t* gl2;
 };
 
-__global__ void __launch_bounds__(kCanonTPB, 2) canon_kernel(CanonArgs a) {
-  extern __shared__ __align__(16) uint8_t s_perm[];
-  // the GL2 table, rows padded from 49 to kGl2Row bytes
-  for (int i = threadIdx.x; i < kGl2Order * kN; i += blockDim.x) {
-    const int m = i / kN;
-    s_perm[m * kGl2Row + (i - m * kN)] = __ldg(a.gl2 + i);
+__global__ void __launch_bounds__(kCanonTPB) canon_kernel(CanonArgs a) {
+  __shared__ CanonTable tab;
+  __shared__ CanonScratch scratch[kCanonSets];
+  {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(&g_canon_table);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(&tab);
+    for (int i = threadIdx.x; i < int(sizeof(CanonTable) / 4); i += kCanonTPB) dst[i] = src[i];
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const int warps_per_block = blockDim.x >> 5;
-  const int n_warps = gridDim.x * warps_per_block;
-  for (int s = blockIdx.x * warps_per_block + (threadIdx.x >> 5); s < a.n; s += n_warps) {
+  const int d = lane & 7;
+  const int group = threadIdx.x >> 3;
+  // The warp's first set decides, so all 32 lanes stay in the loop.
+  for (int first = blockIdx.x * kCanonSets + (threadIdx.x >> 5) * 4; first < a.n;
+       first += gridDim.x * kCanonSets) {
+    const int s = first + (lane >> 3);
     uint64_t S = 0ull;
     bool bad = false;
-    if (a.sets) {
-      const int k = a.k;
-      const int32_t* row = a.sets + size_t(s) * size_t(k);
-      const int i_a = lane < k ? row[lane] : 0;
-      const int i_b = lane + 32 < k ? row[lane + 32] : 0;
-      const bool bad_a = lane < k && (i_a < 0 || i_a >= kN);
-      const bool bad_b = lane + 32 < k && (i_b < 0 || i_b >= kN);
-      uint64_t mine = 0ull;
-      if (lane < k && !bad_a) mine |= 1ull << i_a;
-      if (lane + 32 < k && !bad_b) mine |= 1ull << i_b;
-      const uint32_t lo = __reduce_or_sync(0xffffffffu, uint32_t(mine));
-      const uint32_t hi = __reduce_or_sync(0xffffffffu, uint32_t(mine >> 32));
-      S = uint64_t(lo) | (uint64_t(hi) << 32);
-      bad = __any_sync(0xffffffffu, bad_a || bad_b) || __popcll(S) != k;
-    } else if (a.expand) {
-      const uint64_t parent = a.masks[s / kN] & kMask49;
-      const int p = s % kN;
-      S = (parent >> p & 1ull) ? 0ull : (parent | (1ull << p));
-    } else {
-      S = a.masks[s] & kMask49;
+    if (s < a.n) {
+      if (a.sets) {
+        const int32_t* row = a.sets + size_t(s) * size_t(a.k);
+        for (int i = d; i < a.k; i += 8) {
+          const int x = row[i];
+          if (x < 0 || x >= kN) bad = true;
+          else S |= 1ull << x;
+        }
+      } else if (a.expand) {
+        const uint64_t parent = a.masks[s / kN] & kMask49;
+        const int p = s % kN;
+        S = (parent >> p & 1ull) ? 0ull : (parent | (1ull << p));
+      } else {
+        S = a.masks[s] & kMask49;
+      }
     }
-    if (bad || S == 0ull) {
-      if (lane == 0) {
+    if (a.sets) {
+      // the lanes' points joined; a repeated index leaves fewer than k
+      for (int o = 4; o > 0; o >>= 1) {
+        S |= __shfl_xor_sync(0xffffffffu, S, o);
+        bad |= __shfl_xor_sync(0xffffffffu, int(bad), o) != 0;
+      }
+      bad |= s < a.n && __popcll(S) != a.k;
+    }
+    if (bad) S = 0ull;
+    const uint64_t best = canon_mask_groups(lane, S, tab, scratch[group]);
+    if (d == 0 && s < a.n) {
+      if (S == 0ull) {
         a.out_mask[s] = 0ull;
         if (a.out_lo) a.out_lo[s] = ~0ull;
         if (a.out_hi) a.out_hi[s] = ~0ull;
         if (bad && a.status) atomicCAS(a.status, 0, TG_ERR_BAD_INPUT);
+      } else {
+        a.out_mask[s] = best;
+        if (a.out_lo || a.out_hi) {
+          uint64_t lo, hi;
+          key_from_mask(best, lo, hi);
+          if (a.out_lo) a.out_lo[s] = lo;
+          if (a.out_hi) a.out_hi[s] = hi;
+        }
       }
-      continue;
-    }
-    const uint64_t best = canon_mask_warp_min<false, kGl2Row>(lane, S, s_perm);
-    if (lane == 0) {
-      a.out_mask[s] = best;
-      uint64_t lo, hi;
-      key_from_mask(best, lo, hi);
-      if (a.out_lo) a.out_lo[s] = lo;
-      if (a.out_hi) a.out_hi[s] = hi;
     }
   }
 }
 
-static bool g_canon_attr[64] = {false};
-
-int run_canonical(int device, int sm_count, const uint8_t* d_gl2, const int32_t* d_sets,
-                  const uint64_t* d_masks, int n, int k, uint64_t* d_out_mask,
-                  uint64_t* d_lo, uint64_t* d_hi, int32_t* d_status, cudaStream_t s,
-                  int expand) {
+int run_canonical(int sm_count, const int32_t* d_sets, const uint64_t* d_masks, int n, int k,
+                  uint64_t* d_out_mask, uint64_t* d_lo, uint64_t* d_hi, int32_t* d_status,
+                  cudaStream_t s, int expand) {
   if (n <= 0) return TG_OK;
-  if (!g_canon_attr[device]) {
-    cudaError_t e = cudaFuncSetAttribute(canon_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kGl2SharedBytes);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(canon_kernel)");
-    g_canon_attr[device] = true;
-  }
-  CanonArgs a{d_sets, d_masks, expand, n, k, d_out_mask, d_lo, d_hi, d_status, d_gl2};
-  const int warps_needed = n;
-  int grid = sm_count * 2;
-  const int max_grid = (warps_needed + (kCanonTPB / 32) - 1) / (kCanonTPB / 32);
-  if (grid > max_grid) grid = max_grid;
-  canon_kernel<<<grid, kCanonTPB, kGl2SharedBytes, s>>>(a);
+  CanonArgs a{d_sets, d_masks, expand, n, k, d_out_mask, d_lo, d_hi, d_status};
+  const int grid = min((n + kCanonSets - 1) / kCanonSets, sm_count * 16);
+  canon_kernel<<<grid, kCanonTPB, 0, s>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "canon_kernel launch");
   return TG_OK;

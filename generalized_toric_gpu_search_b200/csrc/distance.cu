@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <cstdio>
 
+#include "canon_form.cuh"
 #include "common.cuh"
 #include "distance.cuh"
 #include "serve.cuh"

@@ -75,10 +75,11 @@ __device__ __forceinline__ unsigned long long ent_pack(unsigned int st, int mz, 
          (static_cast<unsigned long long>(mz & 0xFF) << 48) | id;
 }
 
-// AGL2(F7) canonical mask of S (popcount >= 1), computed by one warp with the
-// GL2 point table read through L1 (the anchored minimum of canonical.cu).
-__device__ uint64_t canon_mask_warp(int lane, uint64_t S, const uint8_t* gl2) {
-  return canon_mask_warp_min<true>(lane, S, gl2);
+// AGL2(F7) canonical mask of S (popcount >= 1) by one warp: its four lane
+// groups compute the same set (and write the same lists).
+__device__ __noinline__ uint64_t canon_mask_warp(int lane, uint64_t S) {
+  __shared__ CanonScratch s_canon[kSrvTPB / 32];
+  return canon_mask_groups(lane, S, g_canon_table, s_canon[threadIdx.x >> 5]);
 }
 
 __device__ __forceinline__ int srv_stage_level(int st) { return st >> 1; }
@@ -328,7 +329,7 @@ __device__ void srv_prepare(const SrvArgs& a, int lane, unsigned int req, uint8_
       __reduce_or_sync(0xffffffffu, lane < k && my >= 32 ? 1u << (my - 32) : 0u);
   const uint64_t S = uint64_t(lo) | (uint64_t(hi) << 32);
   if (k >= 1 && __popcll(S) == k && a.table_cap) {
-    const uint64_t key = canon_mask_warp(lane, S, a.tab.gl2);
+    const uint64_t key = canon_mask_warp(lane, S);
     int outcome = 0;  // 0: no dedup (table full), 1: leader, 2: hit
     unsigned long long v = 0ull, ts = 0ull;
     if (lane == 0) {

@@ -264,7 +264,6 @@ int tg_server_create(tg_context* ctx, const tg_server_params* p, void* d_arena,
   a.life_ns = static_cast<unsigned long long>(q.life_ms) * 1000000ull;
   a.tab.M = ctx->d_M;
   a.tab.Mp = ctx->d_Mp;
-  a.tab.gl2 = ctx->d_gl2;
   e = cudaStreamCreateWithFlags(&srv->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&srv->aux, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMemsetAsync(srv->d_arena, 0, L.d_total, srv->aux);
