@@ -299,6 +299,10 @@ static int bind_distance(tg_context* ctx, const tg_distance_params* p, const int
   a.is_tasks_per_thread = p->is_tasks_per_thread > 0 ? p->is_tasks_per_thread : 4;
   a.is_max_task_units = p->is_max_task_units > 0 ? p->is_max_task_units : 49;
   bind_workspace(a, L, d_workspace);
+  // Exact batches of the toric matrix whose information sets start at k = 2
+  // (by default and by request) go to the toric walk as a whole: it was the
+  // faster one at every size and k measured, 1 to 40,000 sets of k = 6 to 18.
+  if (ctx->is_toric && L.is_min_k == 2 && p->k_max >= 2) tw_bind(a, ctx->sm_count);
   return TG_OK;
 }
 
@@ -451,6 +455,7 @@ int tg_max_zeros_witness(tg_context* ctx, const tg_distance_params* p, const int
   uint8_t* b = static_cast<uint8_t*>(d_workspace);
   DistArgs a2 = a1;
   bind_workspace(a2, W.p2, b + W.off2);
+  a2.tw = 0;  // the witness pass records codewords: the general walk
   a2.sample_count = 0;
   a2.td_default = 1;
   a2.target = reinterpret_cast<int32_t*>(b + W.td2);

@@ -35,6 +35,7 @@
 //    codeword.
 #include <algorithm>
 #include <cstdio>
+#include <vector>
 
 #include "canon_form.cuh"
 #include "common.cuh"
@@ -77,6 +78,8 @@ int upload_field_tables(int device) {
   e = cudaMemcpyToSymbol(c_binom, binom, sizeof(binom));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_pow7, pow7, sizeof(pow7));
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyToSymbol(c_binom)");
+  const int st = tw_upload_tables();
+  if (st) return st;
   g_tables_ready[device] = true;
   return TG_OK;
 }
@@ -138,7 +141,9 @@ WsLayout ws_layout(const tg_distance_params& p) {
   const size_t n_is = infoset ? n : 0;
   L.is_stride = infoset ? infoset_rows(L.is_min_k, kmax) * kIsVecPerRow : 0;
   L.is_hdr = off;   off = align256(off + (infoset ? sizeof(IsHeader) : 0));
-  L.is_rows = off;  off = align256(off + n * size_t(L.is_stride) * sizeof(V6));
+  L.is_rows = off;
+  off = align256(off + std::max(n * size_t(L.is_stride) * sizeof(V6),
+                                infoset ? tw_region_bytes(int(n), kmax) : 0));
   L.is_units = off; off = align256(off + n_is * sizeof(uint64_t));
   L.is_off = off;   off = align256(off + (infoset ? n + 1 : 0) * sizeof(uint64_t));
   L.is_best = off;  off = align256(off + n_is * sizeof(int32_t));
@@ -839,8 +844,16 @@ __global__ void __launch_bounds__(kTPB) walk_sampled_kernel(DistArgs a) {
 }  // namespace tg
 
 #include "infoset_kernel.cuh"
+#include "toric_walk.cuh"
 
 namespace tg {
+
+size_t tw_region_bytes(int n, int k_max) { return tw_layout(n, k_max).end; }
+
+void tw_bind(DistArgs& a, int sm_count) {
+  a.tw = 1;
+  a.tw_ctas = kTwCtasPerSm * sm_count;
+}
 
 // ---------------------------------------------------------------------------
 // Host launcher
@@ -901,6 +914,17 @@ int run_prepare(const DistArgs& args, cudaStream_t s) {
   const bool sampled = args.sample_count > 0;
   cudaError_t e = cudaMemsetAsync(args.hdr, 0, sizeof(WsHeader), s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(header)");
+  if (args.tw) {
+    // counters, queue header and queue lie one after the other
+    const TwLayout L = tw_layout(args.n, args.k_max);
+    uint8_t* from = reinterpret_cast<uint8_t*>(args.is_hdr);
+    e = cudaMemsetAsync(from, 0, size_t(reinterpret_cast<uint8_t*>(args.is_rows) - from) + L.state,
+                        s);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(queue)");
+    toric_prep_kernel<<<args.n, kTwPrepThreads, 0, s>>>(args);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? TG_OK : cuda_fail(e, "toric prep launch");
+  }
   const int prep_grid = (args.n + kPrepWarps - 1) / kPrepWarps;
   if (sampled) prep_sampled_kernel<<<prep_grid, kPrepWarps * 32, 0, s>>>(args);
   else prep_exact_kernel<<<prep_grid, kPrepWarps * 32, 0, s>>>(args);
@@ -927,6 +951,12 @@ int run_walk(const DistArgs& args, int sm_count, int blocks_per_sm, int tpb, cud
   const bool sampled = args.sample_count > 0;
   const int grid = sm_count * blocks_per_sm;
   cudaError_t e = cudaSuccess;
+  if (args.tw) {  // no set is left to the enumeration walks
+    if (!(parts & kWalkInfoset)) return TG_OK;
+    toric_walk_kernel<<<args.tw_ctas, kTwThreads, kTwSharedBytes, s>>>(args);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? TG_OK : cuda_fail(e, "toric walk launch");
+  }
   if (parts & kWalkEnumeration) {
     switch (tpb) {
       case 64: e = launch_walk<64>(args.variant, sampled, grid, blocks_per_sm, args, s); break;

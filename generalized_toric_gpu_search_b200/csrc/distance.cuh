@@ -110,6 +110,10 @@ struct DistArgs {
   uint64_t* is_off;              // task offsets of the current level per code position (n + 1)
   int32_t* is_perm;              // code at each position (codes ordered by k)
   int32_t* is_best;              // smallest weight met per code
+  // Toric codes by information sets without launches between the levels
+  // (toric_walk.cuh); its arrays lie in the is_rows region.
+  int tw;                        // 1: every set of the batch takes that path
+  int tw_ctas;                   // CTAs of the walk
   // Witness pass only (NULL otherwise): per code and set the pivot columns
   // (kIsMaxSets words), the witness codewords (49 GF(8) symbols per code, in
   // the original column order) and one claim word per code.
@@ -124,6 +128,9 @@ struct DistArgs {
 constexpr int kEnumInfosetAll = 16;
 
 int upload_field_tables(int device);
+int tw_upload_tables();
+void tw_bind(DistArgs& a, int sm_count);
+size_t tw_region_bytes(int n, int k_max);
 int max_patterns(int H);
 int default_tail_rows(const tg_distance_params& p);
 int infoset_min_k(const tg_distance_params& p);
