@@ -126,7 +126,7 @@ WsLayout ws_layout(const tg_distance_params& p) {
   const int Hmax = kmax > R ? kmax - R : 0;
   L.basis_stride = sampled ? 0 : kmax * 3;
   L.pat_stride = sampled ? 0 : max_patterns(Hmax);
-  L.bitpat_stride = sampled ? kmax * 8 : 0;
+  L.bitpat_stride = sampled ? kmax * 8 : 0;  // (the rows; callers have sized scratch by this)
   size_t off = 0;
   L.hdr = off;      off = align256(off + sizeof(WsHeader));
   L.desc = off;     off = align256(off + n * sizeof(CodeDesc));
@@ -718,132 +718,10 @@ __global__ void __launch_bounds__(kTPB, kMinBlocks) walk_direct_kernel(DistArgs 
   }
 }
 
-// ---------------------------------------------------------------------------
-// Sampled screening (kernel_cuda_bp.py:167-236): work_id = 1..sample_count,
-// poly_id or per-coefficient splitmix64 hashing, bit-exact to the reference.
-// ---------------------------------------------------------------------------
-
-constexpr uint64_t kSampleChunk = 64;  // work ids per task
-
-__global__ void __launch_bounds__(kPrepWarps * 32) prep_sampled_kernel(DistArgs a) {
-  const int w = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int c = blockIdx.x * kPrepWarps + w;
-  if (c >= a.n) return;
-  const int64_t beg = a.off[c];
-  const int64_t klong = a.off[c + 1] - beg;
-  CodeDesc d{};
-  d.set_id = a.set_ids ? a.set_ids[c] : c;
-  d.tmax = kN - (a.target ? a.target[c] : a.td_default);
-  bool ok = klong >= 0 && klong <= a.k_max;
-  const int k = ok ? int(klong) : 0;
-  // Each lane loads up to two indices (k <= 49 < 64).
-  const int i_a = (ok && lane < k) ? a.idx[beg + lane] : 0;
-  const int i_b = (ok && lane + 32 < k) ? a.idx[beg + lane + 32] : 0;
-  const bool bad = __any_sync(0xffffffffu, (ok && lane < k && (i_a < 0 || i_a >= kN)) ||
-                                               (ok && lane + 32 < k && (i_b < 0 || i_b >= kN)));
-  if (!ok || bad) {
-    ok = false;
-    if (lane == 0) report_status(a.hdr, TG_ERR_BAD_INPUT);
-  }
-  uint64_t n_tasks = 0;
-  int result = 0;
-  if (ok && k == 0) {
-    // The reference evaluates the empty message sum, the zero codeword.
-    result = a.sample_count > 0 ? kN : 0;
-  } else if (ok) {
-    V6* T = a.bitpat + size_t(c) * a.bitpat_stride;
-    for (int i = 0; i < k; ++i) {
-      const int row = __shfl_sync(0xffffffffu, i < 32 ? i_a : i_b, i & 31);
-      const uint32_t g_lo = a.tab.M[row * kN + lane];
-      const uint32_t g_hi = lane + 32 < kN ? a.tab.M[row * kN + lane + 32] : 0u;
-      for (int v = 0; v < 8; ++v) {
-        const V6 p = ballot_planes(lane, c_mul[v * 8 + g_lo], c_mul[v * 8 + g_hi]);
-        if (lane == 0) v6_stg(T + i * 8 + v, p);
-      }
-    }
-    n_tasks = (uint64_t(a.sample_count) + kSampleChunk - 1) / kSampleChunk;
-  }
-  if (lane == 0) {
-    d.k = k;
-    d.n_tasks = n_tasks;
-    a.desc[c] = d;
-    a.out[c] = result;
-    a.abort[c] = 0;
-    if (n_tasks) {
-      atomicAdd(&a.hdr->codewords, (unsigned long long)a.sample_count);
-      a.hdr->has_tasks = 1;
-    }
-  }
-}
-
-template <int kTPB>
-__global__ void __launch_bounds__(kTPB) walk_sampled_kernel(DistArgs a) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t total = a.hdr->total_tasks;
-  const uint64_t seed = a.seed;
-  const uint64_t count = uint64_t(a.sample_count);
-  for (;;) {
-    uint64_t t;
-    int c;
-    bool active;
-    if (!claim_task(a, total, lane, t, c, active)) break;
-    if (!active) continue;
-    if (ld_flag(a.abort + c)) {
-      skip_code(a, c);
-      continue;
-    }
-    const CodeDesc d = a.desc[c];
-    const uint64_t j = t - __ldg(a.task_off + c);
-    const V6* T = a.bitpat + size_t(c) * a.bitpat_stride;
-    const int k = d.k;
-    const uint64_t sid = uint64_t(int64_t(d.set_id));
-    const bool poly_mode = 3 * k <= 63;
-    const uint64_t w_beg = j * kSampleChunk + 1;
-    const uint64_t w_end = min(count, (j + 1) * kSampleChunk);
-    int m = 0;
-    bool aborted = false;
-    for (uint64_t wid = w_beg; wid <= w_end; ++wid) {
-      V6 v;
-      v6_zero(v);
-      if (poly_mode) {
-        const uint64_t x = seed ^ (sid * 0x9E3779B97F4A7C15ull) ^ (wid * 0xBF58476D1CE4E5B9ull);
-        uint64_t pid = mod_mersenne(splitmix64(x), 3 * k) + 1ull;
-        for (int i = 0; i < k; ++i) {
-          v6_xor(v, v6_ldg(T + i * 8 + int(pid & 7ull)));
-          pid >>= 3;
-        }
-      } else {
-        const uint64_t xf = seed ^ (sid * 0xD6E8FEB86659FD93ull) ^ (wid * 0xA5A3564E27F8861Full);
-        const int forced = int(splitmix64(xf) % uint64_t(k));
-        const uint64_t base = seed ^ (sid * 0x9E3779B97F4A7C15ull) ^ (wid * 0xBF58476D1CE4E5B9ull);
-        for (int i = 0; i < k; ++i) {
-          int cf = int(splitmix64(base ^ (uint64_t(i + 1) * 0x94D049BB133111EBull)) & 7ull);
-          if (i == forced && cf == 0) cf = 1;
-          v6_xor(v, v6_ldg(T + i * 8 + cf));
-        }
-      }
-      const int wt = __popc(lop3<0xFE>(v.l0, v.l1, v.l2)) + __popc(lop3<0xFE>(v.h0, v.h1, v.h2));
-      const int zeros = kN - wt;
-      if (zeros > d.tmax) {
-        m = max(m, zeros);
-        aborted = true;
-        break;
-      }
-      m = max(m, zeros);
-      if ((wid & 15ull) == 0ull && ld_flag(a.abort + c)) break;
-    }
-    if (m > 0) atomicMax(a.out + c, m);
-    if (aborted) {
-      atomicExch(a.abort + c, 1);
-      skip_code(a, c);
-    }
-  }
-}
-
 }  // namespace tg
 
 #include "infoset_kernel.cuh"
+#include "screen.cuh"
 #include "toric_walk.cuh"
 
 namespace tg {
@@ -864,14 +742,12 @@ constexpr int kIsWalkThreads = 128;
 // Two register budgets per CTA shape: 1024 resident threads per SM (64
 // registers per thread) or 512 (128 registers).
 template <int kTPB>
-static cudaError_t launch_walk(int variant, bool sampled, int grid, int blocks_per_sm,
-                               const DistArgs& args, cudaStream_t s) {
+static cudaError_t launch_walk(int variant, int grid, int blocks_per_sm, const DistArgs& args,
+                               cudaStream_t s) {
   constexpr int kFull = 1024 / kTPB;
   constexpr int kHalf = 512 / kTPB;
   const bool full = blocks_per_sm * kTPB >= 1024;
-  if (sampled) {
-    walk_sampled_kernel<kTPB><<<grid, kTPB, 0, s>>>(args);
-  } else if (variant == TG_VARIANT_HISTOGRAM) {
+  if (variant == TG_VARIANT_HISTOGRAM) {
     if (full) walk_hist_kernel<kTPB, kFull><<<grid, kTPB, 0, s>>>(args);
     else walk_hist_kernel<kTPB, kHalf><<<grid, kTPB, 0, s>>>(args);
   } else {
@@ -926,8 +802,12 @@ int run_prepare(const DistArgs& args, cudaStream_t s) {
     return e == cudaSuccess ? TG_OK : cuda_fail(e, "toric prep launch");
   }
   const int prep_grid = (args.n + kPrepWarps - 1) / kPrepWarps;
-  if (sampled) prep_sampled_kernel<<<prep_grid, kPrepWarps * 32, 0, s>>>(args);
-  else prep_exact_kernel<<<prep_grid, kPrepWarps * 32, 0, s>>>(args);
+  if (sampled) {
+    prep_sampled_kernel<<<prep_grid, kPrepWarps * 32, 0, s>>>(args);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? TG_OK : cuda_fail(e, "sampled prep launch");
+  }
+  prep_exact_kernel<<<prep_grid, kPrepWarps * 32, 0, s>>>(args);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "prep kernel launch");
   if (args.is_min_k <= args.k_max) {
@@ -957,11 +837,13 @@ int run_walk(const DistArgs& args, int sm_count, int blocks_per_sm, int tpb, cud
     e = cudaGetLastError();
     return e == cudaSuccess ? TG_OK : cuda_fail(e, "toric walk launch");
   }
-  if (parts & kWalkEnumeration) {
+  if (sampled) {
+    if (parts & kWalkEnumeration) e = launch_screen(args, sm_count, s);
+  } else if (parts & kWalkEnumeration) {
     switch (tpb) {
-      case 64: e = launch_walk<64>(args.variant, sampled, grid, blocks_per_sm, args, s); break;
-      case 256: e = launch_walk<256>(args.variant, sampled, grid, blocks_per_sm, args, s); break;
-      default: e = launch_walk<128>(args.variant, sampled, grid, blocks_per_sm, args, s); break;
+      case 64: e = launch_walk<64>(args.variant, grid, blocks_per_sm, args, s); break;
+      case 256: e = launch_walk<256>(args.variant, grid, blocks_per_sm, args, s); break;
+      default: e = launch_walk<128>(args.variant, grid, blocks_per_sm, args, s); break;
     }
   }
   if (e != cudaSuccess) return cuda_fail(e, "walk kernel launch");
