@@ -366,6 +366,63 @@ int tg_max_zeros(tg_context* ctx, const tg_distance_params* p, const int32_t* d_
   return run_walk(a, ctx->sm_count, bps, tpb, s);
 }
 
+int tg_max_zeros_host(tg_context* ctx, const tg_distance_params* p, const int32_t* h_indices,
+                      int64_t n_indices, const int64_t* h_offsets, const int32_t* h_target,
+                      int32_t* h_out, void* d_buffer, size_t buffer_bytes, void* d_workspace,
+                      size_t workspace_bytes, void* stream) {
+  if (!ctx) return invalid("tg_max_zeros_host: NULL context");
+  int st = check_distance_params(p);
+  if (st) return st;
+  if (n_indices < 0 || !h_indices || !h_offsets || !h_out || !d_buffer ||
+      (reinterpret_cast<uintptr_t>(d_buffer) & 255u))
+    return invalid("tg_max_zeros_host: NULL or unaligned argument");
+  const size_t n = size_t(p->n_sets);
+  const size_t at_idx = align_ws((n + 1) * sizeof(int64_t));
+  const size_t at_td = align_ws(at_idx + size_t(n_indices) * sizeof(int32_t));
+  const size_t at_out = align_ws(at_td + (h_target ? n * sizeof(int32_t) : 0));
+  if (buffer_bytes < at_out + n * sizeof(int32_t)) {
+    set_last_error("tg_max_zeros_host: buffer has %zu bytes, needs %zu", buffer_bytes,
+                   at_out + n * sizeof(int32_t));
+    return TG_ERR_WORKSPACE;
+  }
+  h_out[n] = TG_OK;
+  if (n == 0) return TG_OK;
+  uint8_t* b = static_cast<uint8_t*>(d_buffer);
+  int64_t* d_off = reinterpret_cast<int64_t*>(b);
+  int32_t* d_idx = reinterpret_cast<int32_t*>(b + at_idx);
+  int32_t* d_td = h_target ? reinterpret_cast<int32_t*>(b + at_td) : nullptr;
+  int32_t* d_out = reinterpret_cast<int32_t*>(b + at_out);
+  DistArgs a;
+  st = bind_distance(ctx, p, d_idx, d_off, d_td, nullptr, d_out, d_workspace, workspace_bytes,
+                     true, a);
+  if (st) return st;
+  DeviceGuard g(ctx->device);
+  if (g.error() != cudaSuccess) return cuda_fail(g.error(), "cudaSetDevice");
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaMemcpyAsync(d_off, h_offsets, (n + 1) * sizeof(int64_t),
+                                  cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && n_indices > 0)
+    e = cudaMemcpyAsync(d_idx, h_indices, size_t(n_indices) * sizeof(int32_t),
+                        cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && h_target)
+    e = cudaMemcpyAsync(d_td, h_target, n * sizeof(int32_t), cudaMemcpyHostToDevice, s);
+  if (e != cudaSuccess) st = cuda_fail(e, "tg_max_zeros_host (copies in)");
+  int bps, tpb;
+  launch_shape(p, &bps, &tpb);
+  if (!st) st = run_prepare(a, s);
+  if (!st) st = run_walk(a, ctx->sm_count, bps, tpb, s);
+  if (!st) {
+    e = cudaMemcpyAsync(h_out, d_out, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(h_out + n, &a.hdr->status, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+    if (e != cudaSuccess) st = cuda_fail(e, "tg_max_zeros_host (copies out)");
+  }
+  // also after an error: the caller's buffers are free on return
+  e = cudaStreamSynchronize(s);
+  if (!st && e != cudaSuccess) st = cuda_fail(e, "tg_max_zeros_host");
+  return st;
+}
+
 }  // extern "C"
 
 namespace tg {

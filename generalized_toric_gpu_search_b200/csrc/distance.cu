@@ -127,8 +127,18 @@ WsLayout ws_layout(const tg_distance_params& p) {
   L.basis_stride = sampled ? 0 : kmax * 3;
   L.pat_stride = sampled ? 0 : max_patterns(Hmax);
   L.bitpat_stride = sampled ? kmax * 8 : 0;  // (the rows; callers have sized scratch by this)
+  L.is_min_k = infoset_min_k(p);
+  const bool infoset = L.is_min_k <= kmax;
+  const size_t n_is = infoset ? n : 0;
+  L.is_stride = infoset ? infoset_rows(L.is_min_k, kmax) * kIsVecPerRow : 0;
   size_t off = 0;
+  // the headers and, at the start of is_rows, the toric walk's queue: cleared
+  // together
   L.hdr = off;      off = align256(off + sizeof(WsHeader));
+  L.is_hdr = off;   off = align256(off + (infoset ? sizeof(IsHeader) : 0));
+  L.is_rows = off;
+  off = align256(off + std::max(n * size_t(L.is_stride) * sizeof(V6),
+                                infoset ? tw_region_bytes(int(n), kmax) : 0));
   L.desc = off;     off = align256(off + n * sizeof(CodeDesc));
   L.task_off = off; off = align256(off + (n + 1) * sizeof(uint64_t));
   L.abort = off;    off = align256(off + n * sizeof(int32_t));
@@ -136,14 +146,6 @@ WsLayout ws_layout(const tg_distance_params& p) {
   L.pat_cum = off;  off = align256(off + n * size_t(L.pat_stride) * sizeof(uint64_t));
   L.pat_info = off; off = align256(off + n * size_t(L.pat_stride) * sizeof(uint32_t));
   L.bitpat = off;   off = align256(off + n * size_t(L.bitpat_stride) * sizeof(V6));
-  L.is_min_k = infoset_min_k(p);
-  const bool infoset = L.is_min_k <= kmax;
-  const size_t n_is = infoset ? n : 0;
-  L.is_stride = infoset ? infoset_rows(L.is_min_k, kmax) * kIsVecPerRow : 0;
-  L.is_hdr = off;   off = align256(off + (infoset ? sizeof(IsHeader) : 0));
-  L.is_rows = off;
-  off = align256(off + std::max(n * size_t(L.is_stride) * sizeof(V6),
-                                infoset ? tw_region_bytes(int(n), kmax) : 0));
   L.is_units = off; off = align256(off + n_is * sizeof(uint64_t));
   L.is_off = off;   off = align256(off + (infoset ? n + 1 : 0) * sizeof(uint64_t));
   L.is_best = off;  off = align256(off + n_is * sizeof(int32_t));
@@ -788,15 +790,15 @@ int infoset_last_level(int k_max, int is_toric) {
 int run_prepare(const DistArgs& args, cudaStream_t s) {
   if (args.n <= 0) return TG_OK;
   const bool sampled = args.sample_count > 0;
-  cudaError_t e = cudaMemsetAsync(args.hdr, 0, sizeof(WsHeader), s);
+  // The header; a toric walk's counters, queue header and queue follow it.
+  size_t clear = sizeof(WsHeader);
+  if (args.tw)
+    clear = size_t(reinterpret_cast<uint8_t*>(args.is_rows) -
+                   reinterpret_cast<uint8_t*>(args.hdr)) +
+            tw_layout(args.n, args.k_max).state;
+  cudaError_t e = cudaMemsetAsync(args.hdr, 0, clear, s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(header)");
   if (args.tw) {
-    // counters, queue header and queue lie one after the other
-    const TwLayout L = tw_layout(args.n, args.k_max);
-    uint8_t* from = reinterpret_cast<uint8_t*>(args.is_hdr);
-    e = cudaMemsetAsync(from, 0, size_t(reinterpret_cast<uint8_t*>(args.is_rows) - from) + L.state,
-                        s);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(queue)");
     toric_prep_kernel<<<args.n, kTwPrepThreads, 0, s>>>(args);
     e = cudaGetLastError();
     return e == cudaSuccess ? TG_OK : cuda_fail(e, "toric prep launch");

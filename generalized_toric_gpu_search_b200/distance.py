@@ -18,6 +18,7 @@ maximum as the reference.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import itertools
 import threading
@@ -222,14 +223,23 @@ class DistanceRunner:
             is_max_task_units=c.is_max_task_units,
         )
 
-    def workspace(self, p: _lib.DistanceParams) -> torch.Tensor:
+    def _workspace_bytes(self, p: _lib.DistanceParams) -> int:
         need = ctypes.c_size_t(0)
         _lib.check(_lib.load().tg_distance_workspace_size(ctypes.byref(p), ctypes.byref(need)),
                    "tg_distance_workspace_size")
-        if self._ws is None or self._ws.numel() < need.value:
-            self._ws = torch.empty(max(int(need.value), 256), dtype=torch.uint8,
-                                   device=self.device)
-        return self._ws
+        return max(need.value, 256)
+
+    def held_workspace(self, p: _lib.DistanceParams) -> torch.Tensor | None:
+        """The workspace, if it is large enough for `p`."""
+        ws = self._ws
+        return ws if ws is not None and ws.numel() >= self._workspace_bytes(p) else None
+
+    def workspace(self, p: _lib.DistanceParams) -> torch.Tensor:
+        ws = self.held_workspace(p)
+        if ws is None:
+            ws = self._ws = torch.empty(self._workspace_bytes(p), dtype=torch.uint8,
+                                        device=self.device)
+        return ws
 
     def run(self, p: _lib.DistanceParams, d_indices: torch.Tensor, d_offsets: torch.Tensor,
             d_out: torch.Tensor, d_target: torch.Tensor | None = None,
@@ -372,6 +382,8 @@ class DistanceOracleCUDABP:
         self._stream = torch.cuda.Stream(device=self.device)
         self._lock = threading.Lock()
         self._stage = PinnedBatchStage()
+        self._buffer: torch.Tensor | None = None
+        self._h_out: torch.Tensor | None = None
 
     def _runner_for(self, k_max: int, early_exit: bool) -> DistanceRunner:
         """Launch shape: the fixed config, else the autotuned one for k_max.
@@ -462,7 +474,7 @@ class DistanceOracleCUDABP:
 
     def _evaluate(self, batched_indices, target_distance, sample_count, sample_seed) -> list[int]:
         n = len(batched_indices)
-        with self._lock, torch.cuda.device(self.device):
+        with self._lock, self._on_device():
             staged = self._stage.pack(batched_indices)
             if staged is None:
                 flat, offsets, k_max = pack_sets(batched_indices)
@@ -478,32 +490,60 @@ class DistanceOracleCUDABP:
             if bad:
                 raise ValueError("exponent indices must lie in 0..48")
             per_set_td = not np.isscalar(target_distance)
-            td_arr = None
+            h_td = None
             if per_set_td:
                 td_arr = np.asarray(target_distance, dtype=np.int32)
                 if td_arr.shape != (n,):
                     raise ValueError("target_distance must be an int or one value per set")
-            s = self._stream
-            with torch.cuda.stream(s):
-                d_idx = h_idx.to(self.device, non_blocking=True)
-                d_off = h_off.to(self.device, non_blocking=True)
-                self._stage.mark(s)
-                d_td = None
-                if td_arr is not None:
-                    d_td = torch.from_numpy(td_arr).pin_memory().to(self.device, non_blocking=True)
-                d_out = torch.empty(n, dtype=torch.int32, device=self.device)
-                early = sample_count > 0 or (
-                    bool((td_arr > 1).any()) if td_arr is not None else int(target_distance) > 1)
-                self.runner = self._runner_for(k_max, early)
-                p = self.runner.params(n, k_max, 0 if per_set_td else int(target_distance),
-                                       sample_count if sample_count > 0 else 0, sample_seed)
-                self.runner.run(p, d_idx, d_off, d_out, d_target=d_td, stream=s)
-                h_out = torch.empty(n, dtype=torch.int32, pin_memory=True)
-                h_out.copy_(d_out, non_blocking=True)
-            status = self.runner.status(p, s)  # synchronises the stream
+                early = sample_count > 0 or bool((td_arr > 1).any())
+                h_td = torch.from_numpy(td_arr).pin_memory()
+            else:
+                early = sample_count > 0 or int(target_distance) > 1
+            self.runner = self._runner_for(k_max, early)
+            p = self.runner.params(n, k_max, 0 if per_set_td else int(target_distance),
+                                   sample_count if sample_count > 0 else 0, sample_seed)
+            return self._run_host(p, h_idx, h_off, h_td)
+
+    def _on_device(self):
+        """The oracle's device as the current one (entered only where it is not)."""
+        if torch.cuda.current_device() == self.device.index:
+            return contextlib.nullcontext()
+        return torch.cuda.device(self.device)
+
+    # Device and pinned memory that an oracle keeps between calls; what a
+    # larger batch needs goes back to torch's allocators after the call.
+    KEEP_BYTES = 4 << 20
+
+    def _run_host(self, p, h_idx: torch.Tensor, h_off: torch.Tensor,
+                  h_td: torch.Tensor | None) -> list[int]:
+        """One tg_max_zeros_host call (the caller holds the lock).  It returns
+        with the stream idle, so the buffers are free for the next call."""
+        n, total = p.n_sets, h_idx.numel()
+        need = 8 * (n + 1) + 4 * total + 8 * n + 4 * 256
+        buf, h_out = self._buffer, self._h_out
+        ws = self.runner.held_workspace(p)
+        if ws is None or buf is None or buf.numel() < need:
+            with torch.cuda.stream(self._stream):
+                ws = self.runner.workspace(p)
+                if buf is None or buf.numel() < need:
+                    buf = torch.empty(max(need, 1 << 14), dtype=torch.uint8, device=self.device)
+        if h_out is None or h_out.numel() < n + 1:
+            h_out = torch.empty(max(n + 1, 1 << 10), dtype=torch.int32, pin_memory=True)
+        self._buffer = buf if buf.numel() <= self.KEEP_BYTES else None
+        self._h_out = h_out if 4 * h_out.numel() <= self.KEEP_BYTES else None
+        self.runner.last_params = p
+        _lib.check(
+            _lib.load().tg_max_zeros_host(
+                self.ctx.handle, ctypes.byref(p), h_idx.data_ptr(), total, h_off.data_ptr(),
+                h_td.data_ptr() if h_td is not None else None, h_out.data_ptr(),
+                buf.data_ptr(), buf.numel(), ws.data_ptr(), ws.numel(),
+                self._stream.cuda_stream),
+            "tg_max_zeros_host")
+        got = h_out[:n + 1].numpy().tolist()  # numpy converts faster than torch
+        status = got.pop()
         if status != _lib.TG_OK:
             _lib.check(status, "max_zeros_batch (device)")
-        return h_out.numpy().tolist()  # numpy converts faster than torch
+        return got
 
 
 def init_cuda_oracles_bp(M: np.ndarray) -> tuple[list[DistanceOracleCUDABP], int]:

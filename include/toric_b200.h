@@ -150,6 +150,20 @@ int tg_max_zeros(tg_context* ctx, const tg_distance_params* p,
                  int32_t* d_out, void* d_workspace, size_t workspace_bytes,
                  void* stream);
 
+/* tg_max_zeros from and to host memory, in one call that returns when the
+ * results are there: copies in, kernels, copies out, one synchronisation.
+ *   h_indices, h_offsets, h_target  as d_indices (n_indices of them),
+ *              d_offsets and d_target, in pinned memory
+ *   h_out      pinned, n_sets + 1: the values, then the device status word
+ *   d_buffer   256-byte aligned device memory for the copies: 8 (n_sets + 1),
+ *              4 n_indices, with h_target 4 n_sets, and 4 n_sets bytes, each
+ *              rounded up to 256 */
+int tg_max_zeros_host(tg_context* ctx, const tg_distance_params* p,
+                      const int32_t* h_indices, int64_t n_indices,
+                      const int64_t* h_offsets, const int32_t* h_target,
+                      int32_t* h_out, void* d_buffer, size_t buffer_bytes,
+                      void* d_workspace, size_t workspace_bytes, void* stream);
+
 /* The two halves of tg_max_zeros, for callers that time or capture them
  * separately: _prepare validates the sets, orders rows, builds the bit-sliced
  * bases, the information sets and the task tables (prep + scan kernels);
