@@ -42,9 +42,9 @@
 // 1 to 3 (level 4 of short codes), first stage.  toric_walk_kernel: two
 // persistent CTAs per SM; codes move through their stages on their own (the
 // CTA that counts a stage's last claim opens the next one), so no launch and
-// no barrier separates the levels.  One set of k = 8 takes 101 us by the
-// Python call (193 by the general walk's 31 launches), of k = 14 153 (300),
-// 10,000 sets of k = 6..14 3.5 ms (4.3).
+// no barrier separates the levels.  One set of k = 8 takes 60 us by the Python
+// call (190 by the general walk's 31 launches), of k = 14 120 (305), 10,000
+// sets of k = 6..14 2.9 ms (4.3).
 #pragma once
 
 namespace tg {
@@ -381,79 +381,155 @@ __device__ inline void tw_advance(const DistArgs& a, const TwView& v, int lane, 
 
 constexpr int kTwPrepThreads = 128;
 
-// Weights of P + alpha^v g, v = 0..6, min'd into wmin.
-__device__ __forceinline__ int tw_sweep(const V6& P, V6 g, int wmin) {
-#pragma unroll
-  for (int v = 0; v < 7; ++v) {
-    const int lo = __popc(lop3<0xFE>(P.l0 ^ g.l0, P.l1 ^ g.l1, P.l2 ^ g.l2));
-    const int hi = __popc(lop3<0xFE>(P.h0 ^ g.h0, P.h1 ^ g.h1, P.h2 ^ g.h2));
-    wmin = min(wmin, lo + hi);
-    v6_alpha_pow(g, 1);
-  }
-  return wmin;
-}
-
-// The first 32 columns of a vector: alpha times it, and the sum with another.
-struct TwLo {
+// One word's columns of a vector (three planes).
+struct TwCols {
   uint32_t x0, x1, x2;
 };
 
-__device__ __forceinline__ TwLo tw_lo(const V6& g) { return TwLo{g.l0, g.l1, g.l2}; }
+__device__ __forceinline__ TwCols tw_alpha(const TwCols& g) {
+  return TwCols{g.x2, g.x0 ^ g.x2, g.x1};
+}
 
-__device__ __forceinline__ TwLo tw_lo_alpha(const TwLo& g) {
-  V6 t;
-  v6_zero(t);
-  t.l0 = g.x0;
-  t.l1 = g.x1;
-  t.l2 = g.x2;
-  v6_alpha_pow(t, 1);
-  return tw_lo(t);
+__device__ __forceinline__ TwCols tw_sum(const TwCols& a, const TwCols& b) {
+  return TwCols{a.x0 ^ b.x0, a.x1 ^ b.x1, a.x2 ^ b.x2};
+}
+
+__device__ __forceinline__ TwCols tw_mul(const TwCols& a, const TwCols& b) {
+  const uint32_t d3 = (a.x1 & b.x2) ^ (a.x2 & b.x1), d4 = a.x2 & b.x2;
+  return TwCols{(a.x0 & b.x0) ^ d3, (a.x0 & b.x1) ^ (a.x1 & b.x0) ^ d3 ^ d4,
+                (a.x0 & b.x2) ^ (a.x1 & b.x1) ^ (a.x2 & b.x0) ^ d4};
+}
+
+// a / b column by column, a itself where b is 0, and the columns where b is
+// not.  1 / b = b^2 b^4; squares are linear.
+__device__ __forceinline__ uint4 tw_ratio(const TwCols& a, TwCols b) {
+  const uint32_t nz = b.x0 | b.x1 | b.x2;
+  b.x0 |= ~nz;
+  const TwCols b2{b.x0, b.x2, b.x1 ^ b.x2};
+  const TwCols b4{b2.x0, b2.x2, b2.x1 ^ b2.x2};
+  const TwCols w = tw_mul(a, tw_mul(b2, b4));
+  return make_uint4(w.x0, w.x1, w.x2, nz);
+}
+
+// Sweeps over the last coefficient: the seven codewords P + alpha^v Z, from
+// P / Z.  A column of it names the v that makes a zero there, so a codeword and
+// word of columns take one LOP3 and one POPC (by planes of P + alpha^v Z three
+// and one, which bound the sweep by the ALU); where Z is 0 the column is P's
+// own.  Row r / row z for all r < z is laid out once per code.
+// Whole calls: 4,000 sets of k = 8 237 -> 201 us, of k = 10 515 -> 454, 39,000
+// of k = 10 3.93 -> 3.40 ms, 10,000 of k = 6..14 2.95 -> 2.80; a lone set the
+// same 66 us.
+struct TwRatio {
+  uint4 lo, hi;
+};
+
+__device__ __forceinline__ TwCols tw_cols(const uint4& w) { return TwCols{w.x, w.y, w.z}; }
+
+// The columns where P + alpha^v Z is not 0 for any v, or only for one v.
+__device__ __forceinline__ int tw_own(const TwCols& g, uint32_t nz) {
+  return __popc(lop3<0xFE>(g.x0, g.x1, g.x2) | nz);
+}
+
+__device__ __forceinline__ TwCols tw_mask(const TwCols& g, uint32_t nz) {
+  return TwCols{g.x0 & nz, g.x1 & nz, g.x2 & nz};
+}
+
+// Most zeros that one v makes (g masked).
+__device__ __forceinline__ int tw_most(const TwCols& g) {
+  int most = __popc(lop3<sel_lut(1)>(g.x0, g.x1, g.x2));
+  most = max(most, __popc(lop3<sel_lut(2)>(g.x0, g.x1, g.x2)));
+  most = max(most, __popc(lop3<sel_lut(3)>(g.x0, g.x1, g.x2)));
+  most = max(most, __popc(lop3<sel_lut(4)>(g.x0, g.x1, g.x2)));
+  most = max(most, __popc(lop3<sel_lut(5)>(g.x0, g.x1, g.x2)));
+  most = max(most, __popc(lop3<sel_lut(6)>(g.x0, g.x1, g.x2)));
+  return max(most, __popc(lop3<sel_lut(7)>(g.x0, g.x1, g.x2)));
+}
+
+template <int kV>
+__device__ __forceinline__ int tw_zeros(const TwCols& g, const TwCols& h) {
+  return __popc(lop3<sel_lut(kV)>(g.x0, g.x1, g.x2)) + __popc(lop3<sel_lut(kV)>(h.x0, h.x1, h.x2));
+}
+
+// Least weight over all columns.
+__device__ __forceinline__ int tw_least(const TwCols& lo, const TwCols& hi, uint32_t nz_lo,
+                                        uint32_t nz_hi) {
+  const TwCols g = tw_mask(lo, nz_lo), h = tw_mask(hi, nz_hi);
+  int most = tw_zeros<1>(g, h);
+  most = max(most, tw_zeros<2>(g, h));
+  most = max(most, tw_zeros<3>(g, h));
+  most = max(most, tw_zeros<4>(g, h));
+  most = max(most, tw_zeros<5>(g, h));
+  most = max(most, tw_zeros<6>(g, h));
+  most = max(most, tw_zeros<7>(g, h));
+  return tw_own(lo, nz_lo) + tw_own(hi, nz_hi) - most;
 }
 
 // Codes of at most this many rows have their level 4 done by toric_prep_kernel
 // (1.7e5 codewords at k = 12, 3.4e5 at k = 14), for which the walk's bit rows
 // and its round trips cost more than the codewords: 10,000 sets of k = 6..14
-// 3.7 ms without, 3.2 up to 12, 2.95 up to 14; 2,000 of k = 15 are slower with
-// it (1.08 ms, 0.99).  A lone code of k = 14 is better off with all CTAs on it
-// (0.15 ms, 0.19), so the limit is lower where the codes do not fill the chip.
+// 3.13 ms up to 13, 2.89 up to 14, 2.90 up to 16.  A lone code of k = 14 is
+// better off with all CTAs on it (0.13 ms, 0.15), so the limit is lower where
+// the codes do not fill the chip (11: 40 sets of k = 14 0.225 ms, 12: 0.203).
 constexpr int kTwPrepK = 12, kTwPrepKBig = 14;
 
-// Least weight, below wmin, of the codewords of a stage of level 4: supports by
-// sweeps over the last coefficient, 49 codewords a unit.  The first 32 columns
-// and the 4 on E rule out most; the others are weighed whole.
-__device__ __forceinline__ int tw_level4(const V6* rows, int k, const TwStage& st, int wmin,
+// Up to this many rows level 4 counts all columns at once.  The best weights of
+// short codes let too many sweeps past the first 32 columns, whose second count
+// holds up the warp; from 11 rows on few pass.  4,000 sets: k = 9 282 us by the
+// first columns, 257 whole; k = 10 476 and 455; k = 11 1095 and 1116.
+constexpr int kTwWholeK = 10;
+
+// Least weight, below wmin, of the codewords of a stage of level 4: seven
+// sweeps a unit.  kWhole: all columns are counted.  Else the first 32 and the 4
+// on E rule out most, and what they leave is counted whole after the sweeps.
+template <bool kWhole>
+__device__ __forceinline__ int tw_level4(const TwRatio* ratio, int k, const TwStage& st, int wmin,
                                          int stop, int tid) {
   const int picks = 4 - st.forced(), m = k - st.avoid() - st.forced();
   const uint32_t units = 7u * static_cast<uint32_t>(c_binom[m][picks]);
+  const auto pick = [&](uint32_t i) {
+    return i < units ? __ldg(g_tw_comb + tw_comb_off(picks) + i / 7u) : 0u;
+  };
+  uint32_t next = pick(tid);
   for (uint32_t i = tid; i < units && wmin > stop; i += kTwPrepThreads) {
-    const uint32_t pick = i / 7u, s = i - 7u * pick;
-    const uint32_t r = __ldg(g_tw_comb + tw_comb_off(picks) + pick);
-    const V6& Q = rows[r & 31u];
-    const V6& X = rows[(r >> 5) & 31u];
-    const V6& Y = rows[(r >> 10) & 31u];
-    const V6& Z = rows[picks == 4 ? r >> 15 : uint32_t(k - 1)];
-    V6 x = X;
-    v6_alpha_pow(x, int(s));
-    TwLo y = tw_lo(Y), z[7];
-    z[0] = tw_lo(Z);
+    const uint32_t s = i % 7u, r = next;
+    next = pick(i + kTwPrepThreads);  // on its way during the sweeps
+    const uint32_t rz = picks == 4 ? r >> 15 : uint32_t(k - 1);
+    const TwRatio* by_z = ratio + rz * (rz - 1u) / 2u;
+    const TwRatio &Q = by_z[r & 31u], &X = by_z[(r >> 5) & 31u], &Y = by_z[(r >> 10) & 31u];
+    const uint32_t nz_lo = Q.lo.w, nz_hi = Q.hi.w;
+    const auto head = [&](const uint4& q, TwCols x) {
+      for (uint32_t e = 0; e < s; ++e) x = tw_alpha(x);
+      return tw_sum(tw_cols(q), x);
+    };
+    const TwCols p = head(Q.lo, tw_cols(X.lo));
+    TwCols y = tw_cols(Y.lo);
+    if constexpr (kWhole) {
+      const TwCols ph = head(Q.hi, tw_cols(X.hi));
+      TwCols yh = tw_cols(Y.hi);
 #pragma unroll
-    for (int v = 1; v < 7; ++v) z[v] = tw_lo_alpha(z[v - 1]);
-    const TwLo p{Q.l0 ^ x.l0, Q.l1 ^ x.l1, Q.l2 ^ x.l2};
-#pragma unroll 1
-    for (int t = 0; t < 7; ++t) {
-      const TwLo g{p.x0 ^ y.x0, p.x1 ^ y.x1, p.x2 ^ y.x2};
-      int lo = kN;
-#pragma unroll
-      for (int v = 0; v < 7; ++v)
-        lo = min(lo, __popc((g.x0 ^ z[v].x0) | (g.x1 ^ z[v].x1) | (g.x2 ^ z[v].x2)));
-      if (lo + 4 < wmin) {
-        V6 P = Q, yy = Y;
-        v6_alpha_pow(yy, t);
-        v6_xor(P, x);
-        v6_xor(P, yy);
-        wmin = tw_sweep(P, Z, wmin);
+      for (int t = 0; t < 7; ++t) {
+        wmin = min(wmin, tw_least(tw_sum(p, y), tw_sum(ph, yh), nz_lo, nz_hi));
+        y = tw_alpha(y);
+        yh = tw_alpha(yh);
       }
-      y = tw_lo_alpha(y);
+    } else {
+      uint32_t light = 0u;  // bit t: one of the seven codewords may be lighter
+#pragma unroll
+      for (int t = 0; t < 7; ++t) {
+        const TwCols g = tw_sum(p, y);
+        if (tw_own(g, nz_lo) - tw_most(tw_mask(g, nz_lo)) + 4 < wmin) light |= 1u << t;
+        y = tw_alpha(y);
+      }
+      if (light) {
+        const TwCols ph = head(Q.hi, tw_cols(X.hi));
+        TwCols yh = tw_cols(Y.hi);  // y is back at alpha^7 = 1
+#pragma unroll 1
+        for (; light; light >>= 1) {
+          if (light & 1u) wmin = min(wmin, tw_least(tw_sum(p, y), tw_sum(ph, yh), nz_lo, nz_hi));
+          y = tw_alpha(y);
+          yh = tw_alpha(yh);
+        }
+      }
     }
   }
   return wmin;
@@ -461,12 +537,14 @@ __device__ __forceinline__ int tw_level4(const V6* rows, int k, const TwStage& s
 
 __global__ void __launch_bounds__(kTwPrepThreads) toric_prep_kernel(DistArgs a) {
   __shared__ __align__(16) V6 s_rows[kMaxExactK];
+  __shared__ TwRatio s_ratio[kMaxExactK * (kMaxExactK - 1) / 2];
   __shared__ int s_min[kTwPrepThreads / 32];
   __shared__ int s_walk;
   const TwView view = tw_view(a);
   const int c = blockIdx.x;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
+  uint32_t pair = __ldg(g_tw_comb + tw_comb_off(2) + tid);  // here by the end of the elimination
   const int64_t beg = a.off[c];
   const int64_t klong = a.off[c + 1] - beg;
   const bool ok_k = klong >= 0 && klong <= a.k_max;
@@ -546,40 +624,43 @@ __global__ void __launch_bounds__(kTwPrepThreads) toric_prep_kernel(DistArgs a) 
   __syncthreads();
   if (!s_walk) return;
 
-  // Levels 1 to 3: rows, sweeps over pairs, seven sweeps per triple; the
-  // triples first, so the short units even out the threads' loads.
   const int n1 = k, n2 = k * (k - 1) / 2, n3 = k * (k - 1) * (k - 2) / 6;
+  const auto triple = [&](int u) {
+    return u < n3 ? __ldg(g_tw_comb + tw_comb_off(3) + u) : 0u;
+  };
+  uint32_t next = triple(tid);
+  for (int i = tid; i < n2; i += kTwPrepThreads) {
+    if (i != tid) pair = __ldg(g_tw_comb + tw_comb_off(2) + i);
+    const V6 &A = s_rows[pair & 31u], &Z = s_rows[pair >> 5];
+    s_ratio[i].lo = tw_ratio(TwCols{A.l0, A.l1, A.l2}, TwCols{Z.l0, Z.l1, Z.l2});
+    s_ratio[i].hi = tw_ratio(TwCols{A.h0, A.h1, A.h2}, TwCols{Z.h0, Z.h1, Z.h2});
+  }
+  __syncthreads();
+
+  // Levels 1 to 3: seven sweeps per triple, one per pair, rows; the triples
+  // first, so the short units even out the threads' loads.
   int wmin = kN + 1;
-  for (int u = n1 + n2 + n3 - 1 - tid; u >= 0; u -= kTwPrepThreads) {
-    int r = u;
-    if (r < n1) {
-      const V6 P = s_rows[r];
-      wmin = min(wmin, __popc(P.l0 | P.l1 | P.l2) + __popc(P.h0 | P.h1 | P.h2));
-      continue;
-    }
-    r -= n1;
-    int t = -1;
-    if (r >= n2) {
-      r -= n2;
-      t = 2;
-      while ((t + 1) * t * (t - 1) / 6 <= r) ++t;
-      r -= t * (t - 1) * (t - 2) / 6;
-    }
-    int p = 1;
-    while ((p + 1) * p / 2 <= r) ++p;
-    const int q = r - p * (p - 1) / 2;
-    const V6 Q = s_rows[q];
-    V6 X = s_rows[p];
-    if (t < 0) {
-      wmin = tw_sweep(Q, X, wmin);
-    } else {
-      const V6 G = s_rows[t];
+  for (int u = tid; u < n1 + n2 + n3; u += kTwPrepThreads) {
+    if (u < n3) {
+      const uint32_t rows = next, rz = rows >> 10;
+      next = triple(u + kTwPrepThreads);  // on its way during the sweeps
+      const TwRatio* by_z = s_ratio + rz * (rz - 1u) / 2u;
+      const TwRatio &Q = by_z[rows & 31u], &X = by_z[(rows >> 5) & 31u];
+      const uint32_t nz_lo = Q.lo.w, nz_hi = Q.hi.w;
+      const TwCols lo = tw_cols(Q.lo), hi = tw_cols(Q.hi);
+      TwCols x = tw_cols(X.lo), xh = tw_cols(X.hi);
+#pragma unroll
       for (int s = 0; s < 7; ++s) {
-        V6 P = Q;
-        v6_xor(P, X);
-        wmin = tw_sweep(P, G, wmin);
-        v6_alpha_pow(X, 1);
+        wmin = min(wmin, tw_least(tw_sum(lo, x), tw_sum(hi, xh), nz_lo, nz_hi));
+        x = tw_alpha(x);
+        xh = tw_alpha(xh);
       }
+    } else if (u < n2 + n3) {
+      const TwRatio& Q = s_ratio[u - n3];
+      wmin = min(wmin, tw_least(tw_cols(Q.lo), tw_cols(Q.hi), Q.lo.w, Q.hi.w));
+    } else {
+      const V6& P = s_rows[u - n2 - n3];
+      wmin = min(wmin, __popc(P.l0 | P.l1 | P.l2) + __popc(P.h0 | P.h1 | P.h2));
     }
   }
   const auto least = [&](int x) {
@@ -603,7 +684,9 @@ __global__ void __launch_bounds__(kTwPrepThreads) toric_prep_kernel(DistArgs a) 
       level = l;
       p1 = p;
       words4 = 343ull * c_binom[k - st.avoid() - st.forced()][4 - st.forced()];
-      wmin = least(tw_level4(s_rows, k, st, wmin, tw_stop(k, st, wthr), tid));
+      const int stop = tw_stop(k, st, wthr);
+      wmin = least(k <= kTwWholeK ? tw_level4<true>(s_ratio, k, st, wmin, stop, tid)
+                                  : tw_level4<false>(s_ratio, k, st, wmin, stop, tid));
     }
   }
   if (tid < 32) {
