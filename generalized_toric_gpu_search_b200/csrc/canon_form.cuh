@@ -21,11 +21,13 @@
 // 150 on average over 1 to 49 points) instead of 2016 |S|.
 //
 // Eight lanes serve one set, one direction each in stage 1; the candidates of
-// stage 2 are dealt out to the lanes through a list in shared memory, since
-// most directions keep none.  Integer work on registers and small tables: no
+// stage 2 of a warp's four sets are dealt out to its lanes through one list in
+// shared memory, since most directions keep none and the sets keep uneven
+// numbers (dealt out within each set's eight lanes, 9.8 of a warp's 32 lanes
+// were active per instruction).  Integer work on registers and small tables: no
 // memory traffic but the masks.  1,000,000 sets of 5 to 30 points on a B200:
-// 51.5 ms over all 2016 matrices, 3.1 ms this way; 50,000 sets of 9 points:
-// 0.487 and 0.077 ms.
+// 51.5 ms over all 2016 matrices, 3.11 ms this way with a list per set, 2.12
+// with one per warp; 50,000 sets of 9 points: 487, 71 and 60 us.
 #pragma once
 
 #include "common.cuh"
@@ -77,30 +79,25 @@ constexpr CanonTable make_canon_table() {
 
 __device__ const CanonTable g_canon_table = make_canon_table();
 
-constexpr int kCanonItems = 128;  // candidates listed at a time, per set
+constexpr int kCanonItems = 256;  // candidates listed at a time, per warp
 
-struct CanonScratch {  // shared memory of one set
-  uint64_t img[8];     // S seen from each direction: row l = line l
+struct CanonScratch {  // shared memory of one warp (four sets)
+  uint64_t img[32];             // the sets seen from each direction: row l = line l
+  uint64_t prefix[4];
+  unsigned long long best[4];
+  int p[4];
   uint16_t item[kCanonItems];
 };
 
 __device__ __forceinline__ int mod7(int x) { return x >= 7 ? x - 7 : x; }  // x < 14
 
-__device__ __forceinline__ uint64_t group_min(uint64_t v) {  // over 8 lanes
-  for (int o = 4; o > 0; o >>= 1) {
-    const uint64_t w = __shfl_xor_sync(0xffffffffu, v, o);
-    v = w < v ? w : v;
-  }
-  return v;
-}
-
 // The canonical masks of the four sets of a warp (group = lane / 8; the lanes
-// of a group pass the same S and scratch, S = 0 returns ~0).  The whole warp
+// of a group pass the same S, all the same scratch; S = 0 returns ~0).  The whole warp
 // calls it: loops run until the last group is done, so every shuffle and
 // vote is warp-wide.
 __device__ __forceinline__ uint64_t canon_mask_groups(int lane, uint64_t S, const CanonTable& T,
                                                       CanonScratch& sc) {
-  const int d = lane & 7;
+  const int d = lane & 7, group = lane >> 3;
   // Direction 7: rows as they are.  Direction m < 7: point (a, b) lies on
   // line b + m a at column a.
   uint64_t img = 0ull;
@@ -111,7 +108,7 @@ __device__ __forceinline__ uint64_t canon_mask_groups(int lane, uint64_t S, cons
       img |= T.spread[rot7(uint32_t(S >> (7 * a)) & 127u, s)] << a;
   }
   __syncwarp();
-  sc.img[d] = img;
+  sc.img[lane] = img;
 
   // Candidates (l6, dl) of this direction, bit 6 l6 + dl - 1: the line of row
   // 0, l6 - dl, must hold a point.  Row 6 is decided with them.
@@ -165,7 +162,7 @@ __device__ __forceinline__ uint64_t canon_mask_groups(int lane, uint64_t S, cons
     }
   }
 
-  // Stage 2: (d, l6, dl, mu) of the kept candidates, listed for the group.
+  // Stage 2: (group, d, l6, dl, mu) of the kept candidates, listed for the warp.
   int mine = 0;
   for (uint64_t x = cand; x != 0ull; x &= x - 1ull) {
     const int bit = __ffsll(static_cast<long long>(x)) - 1;
@@ -173,17 +170,19 @@ __device__ __forceinline__ uint64_t canon_mask_groups(int lane, uint64_t S, cons
     const uint32_t pat = uint32_t(img >> (7 * ((l6 + (6 - p) * dl) % 7))) & 127u;
     mine += p ? __popc(T.mus[pat]) : 6;
   }
-  int end = mine;  // inclusive prefix over the group
-  for (int o = 1; o < 8; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, end, o, 8);
-    if (d >= o) end += y;
+  int end = mine;  // inclusive prefix over the warp
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end += y;
   }
-  const int total = __shfl_sync(0xffffffffu, end, 7, 8);
+  const int total = __shfl_sync(0xffffffffu, end, 31);
   const int begin = end - mine;
-  const int inv_p = (0x6325410 >> (4 * p)) & 7;  // 1 / p mod 7 (0 for p = 0)
-  const int top = p > 0 ? p - 1 : 0;               // first row stage 2 decides
-  uint64_t best = ~0ull;
-  for (int base = 0; __any_sync(0xffffffffu, base < total); base += kCanonItems) {
+  if (d == 0) {
+    sc.prefix[group] = prefix;
+    sc.p[group] = p;
+    sc.best[group] = ~0ull;
+  }
+  for (int base = 0; base < total; base += kCanonItems) {
     __syncwarp();
     int at = begin - base;
     for (uint64_t x = cand; x != 0ull; x &= x - 1ull) {
@@ -192,42 +191,47 @@ __device__ __forceinline__ uint64_t canon_mask_groups(int lane, uint64_t S, cons
       const uint32_t pat = uint32_t(img >> (7 * ((l6 + (6 - p) * dl) % 7))) & 127u;
       for (uint32_t m = p ? uint32_t(T.mus[pat]) : 63u; m != 0u; m &= m - 1u, ++at)
         if (at >= 0 && at < kCanonItems)
-          sc.item[at] = uint16_t(d | (l6 << 3) | (dl << 6) | (__ffs(int(m)) << 9));
+          sc.item[at] = uint16_t(d | (l6 << 3) | (dl << 6) | (__ffs(int(m)) << 9) | (group << 12));
     }
     __syncwarp();
     const int n = min(kCanonItems, total - base);
-    for (int i = d; __any_sync(0xffffffffu, i - d < n); i += 8) {
-      if (i < n) {
-        const uint32_t it = sc.item[i];
-        const uint64_t g = sc.img[it & 7u];
-        const int dl = int(it >> 6) & 7;
-        const uint16_t* scale = T.scale + (it >> 9) * 128u;
-        int line = (int(it >> 3 & 7u) + (6 - p) * dl) % 7;
-        const int rho = p ? scale[uint32_t(g >> (7 * line)) & 127u] >> 8 : 0;
-        uint64_t rows = 0ull;  // scaled rows top..0
-        if (p) line = mod7(line + dl);
-        else line = mod7(int(it >> 3 & 7u) + 7 - dl);  // row 0
-        for (int r = top; r >= 0; --r) {
-          rows = (rows << 7) | (scale[uint32_t(g >> (7 * line)) & 127u] & 127u);
-          line = mod7(line + dl);
-        }
-        for (uint32_t pts = uint32_t(rows) & 127u; pts != 0u; pts &= pts - 1u) {
-          const int nu = mod7(8 - __ffs(int(pts)));  // moves the point to column 0
-          const int neg = p ? ((nu + 7 - rho) * inv_p) % 7 : 0;  // -sigma
-          int s = p ? mod7(rho + neg) : nu;
-          uint64_t cur = (prefix << 7) | rot7(uint32_t(rows >> (7 * top)) & 127u, s);
-          if (cur > (best >> (7 * top))) continue;
-          for (int r = top - 1; r >= 0; --r) {
-            s = mod7(s + neg);
-            cur = (cur << 7) | rot7(uint32_t(rows >> (7 * r)) & 127u, s);
-          }
-          best = cur < best ? cur : best;
-        }
+    for (int i = lane; i < n; i += 32) {
+      const uint32_t it = sc.item[i];
+      const uint32_t of = it >> 12;
+      const uint64_t g = sc.img[8u * of + (it & 7u)], pre = sc.prefix[of];
+      const int q = sc.p[of], dl = int(it >> 6) & 7;
+      const int inv_q = (0x6325410 >> (4 * q)) & 7;  // 1 / q mod 7 (0 for q = 0)
+      const int top = q > 0 ? q - 1 : 0;             // first row stage 2 decides
+      const uint16_t* scale = T.scale + ((it >> 9) & 7u) * 128u;
+      int line = (int(it >> 3 & 7u) + (6 - q) * dl) % 7;
+      const int rho = q ? scale[uint32_t(g >> (7 * line)) & 127u] >> 8 : 0;
+      uint64_t rows = 0ull;  // scaled rows top..0
+      if (q) line = mod7(line + dl);
+      else line = mod7(int(it >> 3 & 7u) + 7 - dl);  // row 0
+      for (int r = top; r >= 0; --r) {
+        rows = (rows << 7) | (scale[uint32_t(g >> (7 * line)) & 127u] & 127u);
+        line = mod7(line + dl);
       }
-      best = group_min(best);
+      // what any lane has reached for this set (a late look only prunes less)
+      const uint64_t seen = *reinterpret_cast<volatile unsigned long long*>(&sc.best[of]);
+      uint64_t best = seen;
+      for (uint32_t pts = uint32_t(rows) & 127u; pts != 0u; pts &= pts - 1u) {
+        const int nu = mod7(8 - __ffs(int(pts)));  // moves the point to column 0
+        const int neg = q ? ((nu + 7 - rho) * inv_q) % 7 : 0;  // -sigma
+        int s = q ? mod7(rho + neg) : nu;
+        uint64_t cur = (pre << 7) | rot7(uint32_t(rows >> (7 * top)) & 127u, s);
+        if (cur > (best >> (7 * top))) continue;
+        for (int r = top - 1; r >= 0; --r) {
+          s = mod7(s + neg);
+          cur = (cur << 7) | rot7(uint32_t(rows >> (7 * r)) & 127u, s);
+        }
+        best = cur < best ? cur : best;
+      }
+      if (best < seen) atomicMin(&sc.best[of], static_cast<unsigned long long>(best));
     }
   }
-  return best;
+  __syncwarp();
+  return sc.best[group];
 }
 
 }  // namespace tg

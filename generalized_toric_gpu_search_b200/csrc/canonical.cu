@@ -35,7 +35,7 @@ struct CanonArgs {
 
 __global__ void __launch_bounds__(kCanonTPB) canon_kernel(CanonArgs a) {
   __shared__ CanonTable tab;
-  __shared__ CanonScratch scratch[kCanonSets];
+  __shared__ CanonScratch scratch[kCanonTPB / 32];
   {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(&g_canon_table);
     uint32_t* dst = reinterpret_cast<uint32_t*>(&tab);
@@ -44,7 +44,6 @@ __global__ void __launch_bounds__(kCanonTPB) canon_kernel(CanonArgs a) {
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int d = lane & 7;
-  const int group = threadIdx.x >> 3;
   // The warp's first set decides, so all 32 lanes stay in the loop.
   for (int first = blockIdx.x * kCanonSets + (threadIdx.x >> 5) * 4; first < a.n;
        first += gridDim.x * kCanonSets) {
@@ -76,7 +75,7 @@ __global__ void __launch_bounds__(kCanonTPB) canon_kernel(CanonArgs a) {
       bad |= s < a.n && __popcll(S) != a.k;
     }
     if (bad) S = 0ull;
-    const uint64_t best = canon_mask_groups(lane, S, tab, scratch[group]);
+    const uint64_t best = canon_mask_groups(lane, S, tab, scratch[threadIdx.x >> 5]);
     if (d == 0 && s < a.n) {
       if (S == 0ull) {
         a.out_mask[s] = 0ull;

@@ -75,11 +75,13 @@ __device__ __forceinline__ unsigned long long ent_pack(unsigned int st, int mz, 
          (static_cast<unsigned long long>(mz & 0xFF) << 48) | id;
 }
 
-// AGL2(F7) canonical mask of S (popcount >= 1) by one warp: its four lane
-// groups compute the same set (and write the same lists).
+// AGL2(F7) canonical mask of S (popcount >= 1) by one warp: the first lane
+// group has the set, the others none; the candidates go to all lanes.
 __device__ __noinline__ uint64_t canon_mask_warp(int lane, uint64_t S) {
   __shared__ CanonScratch s_canon[kSrvTPB / 32];
-  return canon_mask_groups(lane, S, g_canon_table, s_canon[threadIdx.x >> 5]);
+  const uint64_t best = canon_mask_groups(lane, lane < 8 ? S : 0ull, g_canon_table,
+                                          s_canon[threadIdx.x >> 5]);
+  return __shfl_sync(0xffffffffu, best, 0);
 }
 
 __device__ __forceinline__ int srv_stage_level(int st) { return st >> 1; }
