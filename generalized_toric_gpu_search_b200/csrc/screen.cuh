@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kScreenThreads) screen_kernel(DistArgs a, uint
   const uint64_t piece = blockIdx.x / a.n;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const CodeDesc d = a.desc[c];
-  if (d.n_tasks == 0 || a.hdr->has_tasks < 0 || ld_flag(a.abort + c)) return;
+  if (d.n_tasks == 0 || a.hdr->has_tasks < 0) return;
   const int k = d.k, groups = screen_groups(k);
   uint32_t* table = screen_raw;
   uint32_t* vec = screen_raw + groups * kScreenGroupWords;  // five words per bit
@@ -133,7 +133,9 @@ __global__ void __launch_bounds__(kScreenThreads) screen_kernel(DistArgs a, uint
       v6_alpha_pow(g, 1);
     }
   }
-  __syncthreads();
+  // Another CTA of the code may set the flag meanwhile: one thread looks at it
+  // for all, since the table below is laid out by every warp or not at all.
+  if (__syncthreads_or(tid == 0 && ld_flag(a.abort + c))) return;
   for (int g = warp; g < groups; g += kScreenThreads / 32) {
     uint32_t x[5] = {0u, 0u, 0u, 0u, 0u};
     for (int b = 0; b < 5 && 5 * g + b < 3 * k; ++b) {
