@@ -80,6 +80,12 @@ def last_infoset_level(k_max: int) -> int:
     return last
 
 
+def takes_toric_walk(k_max: int, enumeration: str) -> bool:
+    """Whether an exact batch of the toric matrix goes to toric_prep_kernel and
+    toric_walk_kernel (the rule of bind_distance, csrc/abi.cu)."""
+    return k_max >= 2 and enumeration in ("auto", "infoset")
+
+
 def launches_per_step(k_max: int, enumeration: str) -> int:
     """Kernels per step: prep_exact, scan_tasks and the enumeration walk; with
     information sets also prep_infoset, order_codes, levels123 (levels 1 to
@@ -798,14 +804,17 @@ def run_b200_arm(args, d: Dist) -> None:
     M = build_eval_matrix()
     ctx = ToricContext(dev, M)
     flat, offsets, kmax = pack_sets(sets)
-    # The launch shape the autotuner picked for this batch's largest k (tuned
-    # here first when the device has no table), with the command line's
-    # orbit-walk overrides.
+    # Exact batches of the toric matrix (k >= 2) take the toric walk, whose shape
+    # is fixed.  The walks over all messages take the shape that a table of this
+    # device holds for the batch's largest k, with the command line's overrides.
     from dataclasses import asdict, replace
 
     from generalized_toric_gpu_search_b200 import autotune
 
-    tuned = autotune.choose(autotune.ensure_table(dev), kmax) if not args.no_autotune else None
+    toric_walk = takes_toric_walk(kmax, args.enumeration)
+    tuned = None
+    if not toric_walk and not args.no_autotune:
+        tuned = autotune.choose(autotune.load_table(_lib.device_info(dev)[3]), kmax)
     cfg = replace(tuned or LaunchConfig(), enumeration=ENUMERATIONS[args.enumeration][0])
     if args.tail_rows:
         cfg = replace(cfg, tail_rows=args.tail_rows)
@@ -975,8 +984,10 @@ def run_b200_arm(args, d: Dist) -> None:
                        "launch": "CUDA graphs: prepare, enumeration walk, information-set walk",
                        "launch_shape": {k_: v for k_, v in asdict(cfg).items()
                                         if k_ not in ("enumeration", "variant")},
-                       "launch_shape_source": ("autotuned for k = %d (0 = library default)"
-                                               % kmax) if tuned else "library defaults",
+                       "launch_shape_source":
+                           "fixed: toric walk, two CTAs per SM" if toric_walk else
+                           "table of this device for k = %d (0 = library default)" % kmax
+                           if tuned else "library defaults",
                        "l2": "256 MiB write between timed steps",
                        "parallelism": f"weak, {d.world} rank(s), no data-path collective"},
             "codes_per_s": d.world * len(sets) / (total_ms / 1e3 / args.steps),

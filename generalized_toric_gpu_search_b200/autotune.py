@@ -1,7 +1,9 @@
 """Per-k launch-shape autotuner of the batched max_zeros kernels.
 
-The information-set walk (the default enumeration for k >= 2) has three
-knobs, tuned per k:
+The general information-set walk has three knobs, tuned per k.  It runs the
+exact batches (k >= 2) of matrices other than the toric one, and the witness
+pass; exact batches of the toric matrix take the toric walk, whose shape is
+fixed, so nothing is tuned for them:
   is_blocks_per_sm     -- resident CTAs of 128 threads per SM (1..5);
   is_tasks_per_thread  -- a level is cut into about this many tasks per
                           resident thread (the equal-cost slice count);
@@ -15,9 +17,9 @@ Codes are not pinned to CTAs: every warp claims 32 tasks at a time from one
 queue, so codes per CTA follow from the task size.  `tune` times every
 candidate on a seeded calibration batch per k and records the fastest in a
 JSON cache keyed by the GPU name; `ensure_table` tunes the information-set
-knobs of the k it lacks (a few seconds), which DistanceOracleCUDABP does at
-first use on a device without a table; `choose` returns the shape for a
-batch by its largest k.
+knobs of the k it lacks (a few seconds), which DistanceOracleCUDABP does for
+a matrix other than the toric one at first use on a device without a table;
+`choose` returns the shape for a batch by its largest k.
 """
 
 from __future__ import annotations
@@ -45,6 +47,11 @@ INFOSET_CANDIDATES = [
 ]
 
 INFOSET_KS = range(6, 16)
+
+# Mark of a table entry whose information-set knobs were timed on the general
+# walk.  Tables may hold entries without it, timed on toric batches: those of a
+# library that sends such batches to the toric walk are noise.
+_WALK_KEY, _WALK = "infoset_walk", "general"
 _SHAPE_KEYS = ("tail_rows", "blocks_per_sm", "threads_per_block", "is_blocks_per_sm",
                "is_tasks_per_thread", "is_max_task_units")
 
@@ -87,14 +94,17 @@ def save_table(device_name: str, table: dict[int, dict], path: Path | None = Non
 def choose(table: dict[int, dict], k_max: int) -> LaunchConfig | None:
     """Shape for a batch whose largest set has k_max rows: the entry of the
     nearest tuned k at or below k_max (work is dominated by the largest k);
-    knobs an entry does not hold keep the library defaults."""
+    knobs an entry does not hold keep the library defaults, and so do
+    information-set knobs that were not timed on the walk that reads them."""
     if not table:
         return None
     ks = sorted(table)
     below = [k for k in ks if k <= k_max]
     k = below[-1] if below else ks[0]
     e = table[k]
-    return LaunchConfig(**{key: int(e[key]) for key in _SHAPE_KEYS if key in e})
+    stale = "infoset_seconds" in e and e.get(_WALK_KEY) != _WALK
+    return LaunchConfig(**{key: int(e[key]) for key in _SHAPE_KEYS
+                           if key in e and not (stale and key.startswith("is_"))})
 
 
 def calibration_sets(k: int, target_codewords: float = 2e10, seed: int = 97) -> list[list[int]]:
@@ -106,10 +116,19 @@ def calibration_sets(k: int, target_codewords: float = 2e10, seed: int = 97) -> 
 
 
 def infoset_calibration_sets(k: int, seed: int = 197) -> list[list[int]]:
-    """Seeded sets of size k for the information-set walk (a few ms a batch)."""
-    n = 4096 if k <= 9 else 1024
+    """Seeded sets of size k for the general information-set walk (up to about
+    25 ms a batch)."""
+    n = 4096 if k <= 9 else 1024 if k <= 11 else 296 if k <= 13 else 148
     rng = np.random.default_rng(seed + k)
     return [sorted(rng.choice(49, k, replace=False).tolist()) for _ in range(n)]
+
+
+def general_walk_matrix() -> np.ndarray:
+    """The toric matrix with its columns shifted by one: codes of the same
+    weights, evaluated by the general walk."""
+    from .tables import build_eval_matrix
+
+    return np.roll(build_eval_matrix(), 1, axis=1)
 
 
 def measure(runner_factory, sets, config: LaunchConfig, reps: int = 2) -> float:
@@ -142,15 +161,15 @@ def tune(device_id: int = 0, ks=range(6, 16), candidates=None, path: Path | None
          verbose: bool = False, walk: str = "orbit") -> dict[int, dict]:
     """Times every candidate shape per k and stores the fastest.  walk
     "orbit" tunes the orbit walk's knobs (enumeration TG_ENUM_ORBIT),
-    "infoset" the information-set walk's (the default enumeration); the
-    knobs of the other walk in a table entry are kept."""
+    "infoset" the general information-set walk's, on a matrix that takes it;
+    the knobs of the other walk in a table entry are kept."""
     from . import _lib
     from .distance import DistanceRunner, ToricContext
     from .tables import build_eval_matrix
 
     infoset = walk == "infoset"
     cands = candidates or (INFOSET_CANDIDATES if infoset else CANDIDATES)
-    ctx = ToricContext(device_id, build_eval_matrix())
+    ctx = ToricContext(device_id, general_walk_matrix() if infoset else build_eval_matrix())
     name = _lib.device_info(device_id)[3]
     table = load_table(name, path)
     for k in ks:
@@ -170,6 +189,8 @@ def tune(device_id: int = 0, ks=range(6, 16), candidates=None, path: Path | None
         entry.update(c_best)
         entry["infoset_seconds" if infoset else "seconds"] = t_best
         entry["n_sets" if not infoset else "infoset_n_sets"] = len(sets)
+        if infoset:
+            entry[_WALK_KEY] = _WALK
         entry["tuned_at"] = time.strftime("%Y-%m-%dT%H:%M:%S")
         table[k] = entry
     save_table(name, table, path)
@@ -184,7 +205,7 @@ def ensure_table(device_id: int = 0, ks=INFOSET_KS, path: Path | None = None) ->
 
     name = _lib.device_info(device_id)[3]
     table = load_table(name, path)
-    missing = [k for k in ks if "is_tasks_per_thread" not in table.get(k, {})]
+    missing = [k for k in ks if table.get(k, {}).get(_WALK_KEY) != _WALK]
     if missing:
         table = tune(device_id, ks=missing, path=path, walk="infoset")
     return table

@@ -43,8 +43,9 @@ class LaunchConfig:
     variant: int = _lib.TG_VARIANT_AUTO
     blocks_per_sm: int = 0
     threads_per_block: int = 0
-    # the information-set walk: CTAs per SM, tasks per resident thread of a
-    # level, largest task in 49-codeword blocks (0 = library defaults 5, 4, 49)
+    # the general information-set walk (matrices other than the toric one, and
+    # witnesses): CTAs per SM, tasks per resident thread of a level, largest
+    # task in 49-codeword blocks (0 = library defaults 5, 4, 49)
     is_blocks_per_sm: int = 0
     is_tasks_per_thread: int = 0
     is_max_task_units: int = 0
@@ -365,13 +366,15 @@ class DistanceOracleCUDABP:
         self.ctx = ToricContext(device_id, M)
         self._fixed = config
         self._table: dict = {}
-        if config is None and autotune:
+        # Exact batches of the toric matrix take a walk of fixed shape, so there
+        # is nothing to tune; the witness pass keeps the library defaults.
+        if config is None and autotune and not self.ctx.is_toric:
             import os
 
             from .autotune import ensure_table, load_table
 
             # A device without a table is tuned at first use (a few seconds),
-            # unless TORIC_B200_AUTOTUNE=0 asks for the library defaults.
+            # unless TORIC_B200_AUTOTUNE=0 asks for what is there.
             if os.environ.get("TORIC_B200_AUTOTUNE", "1") != "0":
                 self._table = ensure_table(device_id)
             else:
@@ -386,10 +389,11 @@ class DistanceOracleCUDABP:
         self._h_out: torch.Tensor | None = None
 
     def _runner_for(self, k_max: int, early_exit: bool) -> DistanceRunner:
-        """Launch shape: the fixed config, else the autotuned one for k_max.
-        The table is tuned on exact batches (every level walked); a sampled
-        batch, or one whose thresholds can end sets early, keeps the library
-        defaults, whose smaller tasks notice an early exit sooner."""
+        """Launch shape: the fixed config, else (matrices other than the toric
+        one) the autotuned one for k_max.  The table is tuned on exact batches
+        (every level walked); a sampled batch, or one whose thresholds can end
+        sets early, keeps the library defaults, whose smaller tasks notice an
+        early exit sooner."""
         cfg = self._fixed
         if cfg is None and not early_exit and self._table:
             from .autotune import choose

@@ -118,7 +118,11 @@ typedef struct tg_distance_params {
   int32_t target_distance; /* used for every set when d_target is NULL       */
   int64_t sample_count;    /* 0 = exact; > 0 = reference sampled screening   */
   uint64_t sample_seed;    /* splitmix64 seed of the sampled mode            */
-  /* Launch shape of the information-set walk (ABI version 2): */
+  /* Launch shape of the general information-set walk (ABI version 2): matrices
+   * other than the toric one, and the witness pass.  Exact batches of the toric
+   * matrix (AUTO or INFOSET, k_max >= 2) take the toric walk, whose shape is
+   * fixed; there these three, tail_rows, variant, blocks_per_sm and
+   * threads_per_block have no effect. */
   int32_t is_blocks_per_sm;    /* CTAs of 128 threads per SM, 1..5; 0 = 5        */
   int32_t is_tasks_per_thread; /* a level is cut into about this many tasks per
                                   resident thread, 1..64; 0 = 4                  */
