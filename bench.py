@@ -40,17 +40,18 @@ METRIC = "GF(8) codewords/s, reference-equivalent (8^k-1 messages per code), bat
 UNIT = "codewords/s"
 WORKLOAD = "batched uneven evaluation: 10,000 seeded random P, |P|~U{6..14}, td=1, exact"
 POPC_PER_CODEWORD = 14.0 / 8.0  # histogram walk: 7 bins x 2 words per 8 codewords
-# information-set walk: per sweep of 7 codewords, 7 selection counts on the
-# low 32 columns plus one count of the zero columns of the swept row (the
-# single-count test; where the threshold allows, the kernel tests pairs of
-# codewords with 4 + 1 counts, so the executed POPC can be lower)
-POPC_PER_CODEWORD_INFOSET = 8.0 / 7.0
-# DRAM traffic of one walk_level_kernel launch (dram__bytes_read.sum +
-# dram__bytes_write.sum) from an ncu capture of part 2 of level 5 of 1000 sets
-# of k = 14 (3.09e9 codewords).  The walk reads each set's tables (7 x 32 B
-# per row) and the task offsets; it is integer-issue bound, and DRAM stays
-# near idle.
-WALK_LEVEL5_DRAM_BYTES = 2.34e6
+# toric_walk_kernel: a carry-save adder over 30 columns' bit rows takes 54 LOP3
+# per 32 codewords (the fewest columns it counts: codes of up to 12 rows count
+# 36 or 42, so the executed LOP3 are more)
+LOP3_PER_CODEWORD_TORIC_WALK = 54.0 / 32.0
+# DRAM traffic of one toric_walk_kernel launch (dram__bytes.sum) from an ncu
+# capture of 1000 sets of k = 14 (4.75e9 codewords): the walk reads each set's
+# tables (112 bytes per row) and keeps everything else on the SM.
+TORIC_WALK_DRAM_BYTES = 2.0e6
+# toric_prep_kernel: per sweep of 7 codewords, 7 counts on the low 32 columns
+# and one of the columns that no coefficient makes zero (the fewest: sweeps over
+# all columns count both words)
+POPC_PER_CODEWORD_TORIC_PREP = 8.0 / 7.0
 
 
 # --enumeration: (TG_ENUM_* value, description)
@@ -87,12 +88,52 @@ def takes_toric_walk(k_max: int, enumeration: str) -> bool:
 
 
 def launches_per_step(k_max: int, enumeration: str) -> int:
-    """Kernels per step: prep_exact, scan_tasks and the enumeration walk; with
-    information sets also prep_infoset, order_codes, levels123 (levels 1 to
+    """Kernels per step of the general walks: prep_exact, scan_tasks and the
+    enumeration walk; with information sets also prep_infoset, order_codes, levels123 (levels 1 to
     3), per level 4..last_infoset_level(k_max) two parts of plan, scan and
     walk each, and finalize_infoset."""
     infoset = enumeration == "infoset" or (enumeration == "auto" and k_max >= 2)
     return 3 + ((4 + 6 * max(0, last_infoset_level(k_max) - 3)) if infoset else 0)
+
+
+def step_launches(k_max: int, enumeration: str) -> int:
+    """Kernels per step of a toric batch: toric_prep_kernel and
+    toric_walk_kernel, or the general walks'."""
+    return 2 if takes_toric_walk(k_max, enumeration) else launches_per_step(k_max, enumeration)
+
+
+def roofline(toric: bool, prep_s: float, enum_s: float, infoset_s: float, prep_codewords: int,
+             paths: dict, pipes: dict, sm_count: int, mhz: float) -> dict:
+    """The dominant kernel of a step against the integer pipe that bounds it:
+    of a toric batch the longer of its two kernels, each with the codewords it
+    evaluates itself, else the walk over all messages."""
+    if not toric:
+        kernel, seconds, codewords = "walk_hist_kernel", enum_s, paths["enumeration_codewords"]
+        pipe, per, note = "popc", POPC_PER_CODEWORD, "14 POPC per 8-codeword histogram"
+    elif infoset_s >= prep_s:
+        kernel, seconds = "toric_walk_kernel", infoset_s
+        codewords = paths["infoset_codewords"] - prep_codewords
+        pipe, per = "lop3", LOP3_PER_CODEWORD_TORIC_WALK
+        note = ("54 LOP3 per 32 codewords, the carry-save adder over 30 columns; the kernel "
+                "executes more (36 or 42 columns for k <= 12, offsets, the bit rows' build)")
+    else:
+        kernel, seconds, codewords = "toric_prep_kernel", prep_s, prep_codewords
+        pipe, per = "popc", POPC_PER_CODEWORD_TORIC_PREP
+        note = ("8 POPC per sweep of 7 codewords over the low 32 columns; the kernel executes "
+                "more (both words up to k = 10 and below level 4)")
+    clocks = sm_count * mhz * 1e6  # SM clocks a second
+    peak = pipes.get(f"{pipe}_per_clk_sm", {"lop3": 64.0, "popc": 16.0}[pipe]) * clocks
+    achieved = per * codewords / seconds
+    traffic = {"traffic": TORIC_WALK_DRAM_BYTES,
+               "traffic_unit": "bytes per launch (ncu, 1000 sets of k = 14, 4.75e9 codewords)"} \
+        if kernel == "toric_walk_kernel" else {}
+    return {"bound": f"int ({pipe.upper()})", "achieved": achieved / 1e12, "peak": peak / 1e12,
+            "unit": f"T{pipe}/s", "frac": achieved / peak, "kernel": kernel,
+            "codewords": int(codewords),
+            "codewords_per_clk_sm": codewords / seconds / clocks,
+            "kernel_share": seconds / (prep_s + enum_s + infoset_s),
+            "note": note + f"; peak = measured {pipe.upper()}/clk/SM x SMs x median SM MHz in "
+                           "the timed region", **traffic}
 
 
 L2_FLUSH_BYTES = 256 << 20
@@ -829,24 +870,32 @@ def run_b200_arm(args, d: Dist) -> None:
     stream = torch.cuda.Stream(device=device)
     flush = torch.empty(L2_FLUSH_BYTES, dtype=torch.uint8, device=device)
 
-    # Three CUDA graphs: prepare (header resets, prep, scans), the enumeration
-    # walk (sets below the information-set threshold) and the information-set
-    # walk, so each walk is timed by its own events.
+    # CUDA graphs for the preparation (header resets, prep; scans of the general
+    # walk), the walk over all messages (which a toric batch does not have) and
+    # the information-set walk, so each is timed by its own events.
     g_prep, g_enum, g_is = (torch.cuda.CUDAGraph() for _ in range(3))
     with torch.cuda.stream(stream):
         runner.run(p, d_idx, d_off, d_out, stream=stream, workspace=ws)  # warm the module
     stream.synchronize()
     with torch.cuda.graph(g_prep, stream=stream, capture_error_mode="thread_local"):
         runner.prepare(p, d_idx, d_off, d_out, stream=stream, workspace=ws)
-    with torch.cuda.graph(g_enum, stream=stream, capture_error_mode="thread_local"):
-        runner.walk(p, d_out, stream=stream, workspace=ws, parts=_lib.TG_WALK_ENUMERATION)
-    with torch.cuda.graph(g_is, stream=stream, capture_error_mode="thread_local"):
-        runner.walk(p, d_out, stream=stream, workspace=ws, parts=_lib.TG_WALK_INFOSET)
+    def walk_graph(graph, parts):
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            runner.walk(p, d_out, stream=stream, workspace=ws, parts=parts)
+        return graph.replay
+
+    def no_walk():
+        pass
+
+    if toric_walk:
+        enum_replay, is_replay = no_walk, walk_graph(g_is, _lib.TG_WALK_INFOSET)
+    else:  # no set of such a batch is left to information sets
+        enum_replay, is_replay = walk_graph(g_enum, _lib.TG_WALK_ENUMERATION), no_walk
 
     def step():
         g_prep.replay()
-        g_enum.replay()
-        g_is.replay()
+        enum_replay()
+        is_replay()
 
     with torch.cuda.stream(stream):
         for _ in range(args.warmup):
@@ -856,6 +905,9 @@ def run_b200_arm(args, d: Dist) -> None:
     tasks, codewords, ref_msgs = runner.counters(stream)
     paths = runner.path_counters(stream)
     stages = runner.stage_counters(stream)
+    with torch.cuda.stream(stream):
+        g_prep.replay()  # what the preparation evaluates by itself
+    prep_codewords = runner.path_counters(stream)["infoset_codewords"]
 
     ev = [[torch.cuda.Event(enable_timing=True) for _ in range(4)] for _ in range(args.steps)]
     clocks = clock_sampler(dev)
@@ -868,9 +920,9 @@ def run_b200_arm(args, d: Dist) -> None:
             ev[i][0].record(stream)
             g_prep.replay()
             ev[i][1].record(stream)
-            g_enum.replay()
+            enum_replay()
             ev[i][2].record(stream)
-            g_is.replay()
+            is_replay()
             ev[i][3].record(stream)
     # Wait with the GIL released, so the clock sampler's thread keeps sampling
     # through the timed region (the step times come from the CUDA events).
@@ -933,28 +985,10 @@ def run_b200_arm(args, d: Dist) -> None:
         plain = {"value": ref_msgs / plain_s, "unit": UNIT, "codes_per_s": len(sets) / plain_s,
                  "sample": "4 sets per k, one launch per set, per-k mean time x k histogram"}
 
-    # Roofline of the dominant kernel: the walk with the larger share of the
-    # step, on the POPC pipe that bounds both walks.
     pipes = measure_pipes(dev) if d.rank == 0 else {}
-    sm_count = ctx.sm_count
-    mhz = clk.get("sm_mhz") or pipes.get("ubench_sm_mhz")
-    peak = pipes.get("popc_per_clk_sm", 16.0) * sm_count * (mhz or 1965.0) * 1e6
-    enum_s, is_s = statistics.mean(enum_ms) / 1e3, statistics.mean(is_ms) / 1e3
-    if is_s >= enum_s:
-        dominant = {"kernel": "walk_level_kernel (two launches per level, one per part, with "
-                              "plan_level_kernel, scan_level_kernel and finalize_infoset_kernel)",
-                    "seconds": is_s, "codewords": paths["infoset_codewords"],
-                    "popc_per_codeword": POPC_PER_CODEWORD_INFOSET,
-                    "note": "8 POPC per 7 codewords (seven zero-selection counts on the low "
-                            "32 columns in the W = P / g domain, one count of g's zero columns); "
-                            "the paired test executes 5 per 7 where the threshold allows, so "
-                            "frac can exceed the XU pipe's measured utilisation"}
-    else:
-        dominant = {"kernel": "walk_hist_kernel", "seconds": enum_s,
-                    "codewords": paths["enumeration_codewords"],
-                    "popc_per_codeword": POPC_PER_CODEWORD,
-                    "note": "1.75 POPC per codeword (14 per 8-codeword histogram)"}
-    achieved = dominant["popc_per_codeword"] * dominant["codewords"] / dominant["seconds"]
+    mhz = clk.get("sm_mhz") or pipes.get("ubench_sm_mhz") or 1965.0
+    roof = roofline(toric_walk, statistics.mean(prep_ms) / 1e3, statistics.mean(enum_ms) / 1e3,
+                    statistics.mean(is_ms) / 1e3, prep_codewords, paths, pipes, ctx.sm_count, mhz)
 
     extra = {}
     ref_gpu = None
@@ -980,8 +1014,10 @@ def run_b200_arm(args, d: Dist) -> None:
             "config": {"workload": WORKLOAD, "n_sets_per_gpu": len(sets),
                        "k_range": [K_LO, K_HI], "target_distance": 1,
                        "enumeration": ENUMERATIONS[args.enumeration][1],
-                       "variant": "histogram", "tail_rows": args.tail_rows or 4,
-                       "launch": "CUDA graphs: prepare, enumeration walk, information-set walk",
+                       "variant": "toric walk" if toric_walk else "histogram",
+                       "tail_rows": None if toric_walk else args.tail_rows or 4,
+                       "launch": "CUDA graphs: preparation, toric walk" if toric_walk else
+                                 "CUDA graphs: preparation, walk over all messages",
                        "launch_shape": {k_: v for k_, v in asdict(cfg).items()
                                         if k_ not in ("enumeration", "variant")},
                        "launch_shape_source":
@@ -999,16 +1035,8 @@ def run_b200_arm(args, d: Dist) -> None:
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h), "ms_per_step": 1e3 * e2e_max / args.steps,
                     "api": "DistanceOracleCUDABP.max_zeros_batch(list of lists, 1)"},
-            "gpu_launches": launches_per_step(kmax, args.enumeration) * args.steps,
-            "roofline": {"bound": "int (POPC pipe)", "achieved": achieved / 1e12,
-                         "peak": peak / 1e12, "unit": "Tpopc/s", "frac": achieved / peak,
-                         "traffic": WALK_LEVEL5_DRAM_BYTES,
-                         "traffic_unit": "bytes per launch of level 5 part 2 (ncu, 1000 "
-                                         "sets of k = 14, 3.09e9 codewords)",
-                         "kernel": dominant["kernel"],
-                         "kernel_share": dominant["seconds"] / (statistics.mean(step_ms) / 1e3),
-                         "note": dominant["note"] + "; peak = measured POPC/clk/SM x SMs x "
-                                 "median SM MHz in the timed region"},
+            "gpu_launches": step_launches(kmax, args.enumeration) * args.steps,
+            "roofline": roof,
             "int_pipes": pipes,
             "clocks": clk,
             "plain_form": plain,
