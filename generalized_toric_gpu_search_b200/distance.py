@@ -514,8 +514,10 @@ class DistanceOracleCUDABP:
             return contextlib.nullcontext()
         return torch.cuda.device(self.device)
 
-    # Device and pinned memory that an oracle keeps between calls; what a
-    # larger batch needs goes back to torch's allocators after the call.
+    # The buffers of the copies (device) and of the results (pinned) are kept
+    # between calls up to this size each; larger ones go back to torch's
+    # allocators after the call.  The workspace and the pinned staging of the
+    # indices stay at the size of the largest batch.
     KEEP_BYTES = 4 << 20
 
     def _run_host(self, p, h_idx: torch.Tensor, h_off: torch.Tensor,
