@@ -32,19 +32,22 @@
 // rare ones that pass are weighed whole.
 //
 // The bounds are the ALU (31 codewords per cycle and SM) and shared memory
-// (128 bytes a cycle: 34); short lists, the build and the batches' own work
-// leave 17 at k = 14 and 15 and 19 at k = 12 in large batches, against 10 to
-// 11 of the walk by POPC (infoset_kernel.cuh).  The same sums as a contraction
-// of +-1 characters on tcgen05 (mxf4, 128 x 112 x 256 tiles) reached 16, and
-// lost it on short lists: a unit's handovers took 9,000 cycles.
+// (128 bytes a cycle: 34).  Whole launches reach 17 to 19 from k = 14 on, 15.5
+// at k = 13, 12 at k = 12 (more columns, shorter lists) and 15 over 10,000 sets
+// of k = 6..14, against 10 of the walk by POPC (infoset_kernel.cuh).  At
+// k = 14 (1,000 sets, 17) the ALU is 80 % busy and the shared-memory pipe 72 %:
+// pairs past the end of a lane's list, the build and the batches' own work take
+// what the bound leaves.  The same sums as a contraction of +-1 characters on
+// tcgen05 were slower: a unit's handovers cost the short lists more than the
+// sums.
 //
 // Kernels.  toric_prep_kernel: one CTA per code, elimination, tables, levels
 // 1 to 3 (level 4 of short codes), first stage.  toric_walk_kernel: two
 // persistent CTAs per SM; codes move through their stages on their own (the
 // CTA that counts a stage's last claim opens the next one), so no launch and
-// no barrier separates the levels.  One set of k = 8 takes 60 us by the Python
-// call (190 by the general walk's 31 launches), of k = 14 120 (305), 10,000
-// sets of k = 6..14 2.9 ms (4.3).
+// no barrier separates the levels.  One set of k = 8 takes 54 us by the Python
+// call (180 by the general walk's 31 launches), of k = 14 122 (304), 10,000
+// sets of k = 6..14 3.1 ms (4.25).
 #pragma once
 
 namespace tg {
@@ -418,7 +421,7 @@ __device__ __forceinline__ uint4 tw_ratio(const TwCols& a, TwCols b) {
 // own.  Row r / row z for all r < z is laid out once per code.
 // Whole calls: 4,000 sets of k = 8 237 -> 201 us, of k = 10 515 -> 454, 39,000
 // of k = 10 3.93 -> 3.40 ms, 10,000 of k = 6..14 2.95 -> 2.80; a lone set the
-// same 66 us.
+// same.
 struct TwRatio {
   uint4 lo, hi;
 };

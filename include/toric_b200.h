@@ -72,9 +72,9 @@ int tg_device_info(int device, int32_t* h_sm_count, int32_t* h_cc_major,
 /* Creates a context on `device` from the 49x49 evaluation matrix M (host,
  * row-major int32, entries 0..7).  Replaces DistanceOracleCUDABP.__init__
  * (kernel_cuda_bp.py:251-258) and CanonicalOracle.__init__
- * (kernel_canon.py:137-148): uploads the matrix tables and the GL2(F7) point
- * permutations once.  When M equals the toric matrix of precompute.py:32-43
- * the context enables the torus-orbit enumeration (see tg_distance_params). */
+ * (kernel_canon.py:137-148): uploads the matrix tables once.  When M equals the
+ * toric matrix of precompute.py:32-43 the context enables the torus-orbit
+ * enumeration and the toric walk (see tg_distance_params). */
 int tg_context_create(int device, const int32_t* h_M, tg_context** out_ctx);
 int tg_context_destroy(tg_context* ctx);
 /* 1 when the context's M is the toric evaluation matrix, else 0. */
@@ -170,7 +170,8 @@ int tg_max_zeros_host(tg_context* ctx, const tg_distance_params* p,
 
 /* The two halves of tg_max_zeros, for callers that time or capture them
  * separately: _prepare validates the sets, orders rows, builds the bit-sliced
- * bases, the information sets and the task tables (prep + scan kernels);
+ * bases, the information sets and the task tables (prep + scan kernels; in a
+ * toric batch one kernel, which also evaluates the first levels);
  * _walk runs the persistent enumeration kernels over the prepared tasks and
  * writes d_out.  Same arguments and workspace as tg_max_zeros; d_out of
  * _prepare receives the values of sets decided without enumeration (k <= 1,
@@ -195,7 +196,8 @@ int tg_max_zeros_walk_part(tg_context* ctx, const tg_distance_params* p,
                            size_t workspace_bytes, void* stream);
 
 /* Last information-set level a batch with sets of at most k_max rows can
- * need (levels 1..3 always run; levels 4..*h_level are launched).  For the
+ * need (levels 1..3 always run; the general walk launches levels 4..*h_level,
+ * in the toric walk each set goes as far as its own bound asks).  For the
  * toric matrix: the smallest L with ceil(49 (L + 1) / k) above the Griesmer
  * cap of a [49, k] code over GF(8), maximised over k <= k_max (9 for
  * k_max = 14); for other matrices k_max.  No
